@@ -34,7 +34,7 @@ def build(with_reference: bool | None = None) -> None:
     subprocess.run(["make", "-s", "-C", _HERE], check=True)
     ref_dir = os.environ.get("KRON_REFERENCE_DIR", "/root/reference")
     if with_reference is None:
-        with_reference = os.path.isdir(ref_dir)
+        with_reference = os.path.exists(os.path.join(ref_dir, "kronmult6_batched.hpp"))
     if with_reference:
         subprocess.run(["make", "-s", "-C", _HERE, "ref", f"REF={ref_dir}"], check=True)
 
