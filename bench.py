@@ -79,11 +79,12 @@ class Workload:
 
     def reference_y(self):
         """The reference's own output for the whole batch, Y from zero
-        (oracle/_ref: the reference's OpenMP build, recursive variant); cached."""
+        (oracle/_ref: the reference's OpenMP build, recursive variant; where it
+        is not built, the oracle's C restatement); cached."""
         if self._yref is None:
             import oracle
 
-            ref = oracle.Reference("recur")
+            ref = oracle.reference_or_restatement()
             self.cpu_setup(self.batch)
             self.cpu_step(ref)
             self._yref = self.cY.copy()
@@ -769,7 +770,7 @@ class XbatchedBig(Workload):
         if self._yref is None:
             import oracle
 
-            ref = oracle.Reference("recur")
+            ref = oracle.reference_or_restatement()
             L, B = self.L, self.batch
             X = self.dX.cpu().numpy()
             Y = np.zeros(L * self.nout)

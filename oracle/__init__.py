@@ -263,3 +263,29 @@ class Reference:
         m_, mp = _i(m)
         n_, np_ = _i(n)
         return self.lib.ref_kron_flops(len(m), mp, np_)
+
+
+class Restatement:
+    """The C restatement behind Reference's calls, for machines where the
+    reference's own build is not there (the golden vectors pin one to the
+    other).  x is preserved; W and subbatch are not used."""
+
+    def kronmult_batched(self, d, n, A, X, Y, W=None):
+        kronmult_batched(d, n, A, X, Y)
+
+    def kronmult_xbatched(self, d, n, a_ptrs, lda, x_ptrs, y_ptrs, w_ptrs, subbatch=0):
+        kronmult_general(d, [n] * d, [n] * d, a_ptrs, [lda] * d, x_ptrs, y_ptrs)
+
+    def kronmult_vbatched_entries(self, shapes, a_ptrs, x_ptrs, y_ptrs, wbytes=1 << 24):
+        for k, s in enumerate(np.asarray(shapes).reshape(-1, 13).tolist()):
+            d = s[0]
+            m, n = s[1:1 + 2 * d:2], s[2:2 + 2 * d:2]
+            kronmult_general(d, m, n, a_ptrs[6 * k:6 * k + d], m, x_ptrs[k:k + 1],
+                             y_ptrs[k:k + 1])
+
+    def kgemm_batched(self, op, mm, nn, kk, alpha, a_ptrs, ldA, b_ptrs, ldB, beta, c_ptrs, ldC):
+        kgemm_batched(op, mm, nn, kk, alpha, a_ptrs, ldA, b_ptrs, ldB, beta, c_ptrs, ldC)
+
+
+def reference_or_restatement():
+    return Reference("recur") if Reference.available("recur") else Restatement()
