@@ -391,7 +391,11 @@ int kron_l2_persist_reset(kron_stream_t stream);
  *                       workspace W, a share of the entries runs
  *                       concurrently on the cluster two-phase kernel (a
  *                       library-owned second stream, joined by events) on
- *                       the SMs the 12-block clusters leave idle
+ *                       the SMs the 12-block clusters leave idle;
+ *                       KRON_SLAB_RESIDENT -- the resident form (FP32), the
+ *                       whole vector in one block's shared memory, no
+ *                       workspace (the built-in choice for large enough
+ *                       batches)
  * kron_autotune times every variant that runs (d, n, precision) on a
  * synthetic batched problem of up to batchCount entries (capped at 1 GiB),
  * records the fastest for that key and returns it (outputs may be NULL).
@@ -423,6 +427,7 @@ int kron_l2_persist_reset(kron_stream_t stream);
 #define KRON_SLAB_WHOLE 2
 #define KRON_SLAB_PLAIN_Y 4
 #define KRON_SLAB_NO_SIDE 8
+#define KRON_SLAB_RESIDENT 16
 
 int kron_autotune(int d, int n, int precision, int batchCount, int *variant, int *param,
                   double *best_us, kron_stream_t stream);

@@ -256,6 +256,8 @@ SLAB_WHOLE = 2
 SLAB_PLAIN_Y = 4
 # "slab" param bit: no side kernel on the SMs the slab clusters leave idle
 SLAB_NO_SIDE = 8
+# "slab" param bit: the resident form (FP32, the vector in one block)
+SLAB_RESIDENT = 16
 
 
 def autotune(d, n, precision="f64", batch=1024, stream=None):

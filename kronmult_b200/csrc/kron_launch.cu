@@ -612,7 +612,12 @@ int launch_variant(Params p, int prec, const Workspace &ws, int variant, int par
   case VAR_BIG:
     return big_supported(p, prec) ? launch_big(p, ws, prec, param, stream)
                                   : KRON_ERROR_NOT_SUPPORTED;
+  case VAR_RESIDENT:
+    return resident_supported(p, prec) ? launch_resident(p, stream)
+                                       : KRON_ERROR_NOT_SUPPORTED;
   case VAR_SLAB:
+    if (param & KRON_SLAB_RESIDENT)
+      return launch_variant(p, prec, ws, VAR_RESIDENT, 0, stream);
     return slab_supported(p, prec) ? launch_slab_side(p, prec, ws, param, stream)
                                     : KRON_ERROR_NOT_SUPPORTED;
   case VAR_SPLIT_TC:
@@ -625,6 +630,11 @@ int launch_variant(Params p, int prec, const Workspace &ws, int variant, int par
   default: return KRON_ERROR_NOT_SUPPORTED;
   }
 }
+
+// FP32 d = 6, n = 6: a block an entry (resident) against a cluster of twelve
+// (slab), microseconds at 20 / 40 / 80 / 4096 entries: 19.8 / 20.5 / 20.9 /
+// 481 against 13.6 / 20.8 / 27.0 / 938.
+static bool prefer_resident(const Params &p) { return p.eend - p.ebase >= 40; }
 
 int launch_kron(Params p, int prec, const Workspace &ws, cudaStream_t stream)
 {
@@ -647,12 +657,16 @@ int launch_kron(Params p, int prec, const Workspace &ws, cudaStream_t stream)
   // default order: the specialised kernels, then the general ones
   // (VAR_SPLIT_TC: split precision at d = 6, n = 8 on the tcgen05 tensor
   // cores, 3.6 ms for 256 entries against 7.5 ms for the CUDA-core split)
-  static const int order[] = {VAR_MMA8, VAR_PIPE,     VAR_SLAB, VAR_SQ,
-                              VAR_GEN,  VAR_BIG,      VAR_SPLIT_TC, VAR_LARGE};
+  // (VAR_RESIDENT: from the batch on that fills the GPU, see prefer_resident)
+  static const int order[] = {VAR_MMA8, VAR_PIPE, VAR_RESIDENT, VAR_SLAB, VAR_SQ,
+                              VAR_GEN,  VAR_BIG,  VAR_SPLIT_TC, VAR_LARGE};
   for (int v : order)
   {
+    if (v == VAR_RESIDENT && !prefer_resident(p))
+      continue;
     if ((v == VAR_MMA8 && std::getenv("KRON_DISABLE_MMA8")) ||
         (v == VAR_PIPE && std::getenv("KRON_DISABLE_PIPE")) ||
+        (v == VAR_RESIDENT && std::getenv("KRON_DISABLE_RESIDENT")) ||
         (v == VAR_SLAB && std::getenv("KRON_DISABLE_SLAB")) ||
         (v == VAR_BIG && std::getenv("KRON_DISABLE_BIG")) ||
         (v == VAR_SPLIT_TC && std::getenv("KRON_DISABLE_SPLIT_TC")))

@@ -58,6 +58,11 @@ long long drain_limit();
 bool big_supported(const Params &p, int prec);
 int launch_big(Params p, const Workspace &ws, int prec, int cluster, cudaStream_t stream);
 
+// Resident kernel for square d = 6, n = 6 in FP32: the vector in one block's
+// shared memory, no workspace (kron_resident.cu).
+bool resident_supported(const Params &p, int prec);
+int launch_resident(const Params &p, cudaStream_t stream);
+
 // Split precision (FP64 data, exact BF16 slice products on the tcgen05 tensor
 // cores) for square d = 6, n = 8 in the batched layout with a workspace W
 // (kron_splittc.cu).
@@ -79,6 +84,8 @@ enum Variant : int
   VAR_LARGE = 6, // two-phase launches through the workspace (param unused)
   VAR_SLAB  = 7, // slab-cluster kernel, no workspace; param: KRON_SLAB_NO_ROTATE
   VAR_SPLIT_TC = 8, // split precision d = 6, n = 8 on the tcgen05 tensor cores
+  VAR_RESIDENT = 10, // FP32 vector resident in one block; in the tuning table it is
+                    // VAR_SLAB with KRON_SLAB_RESIDENT
 };
 
 // Work items of a launch (launch_kron does this before any variant).

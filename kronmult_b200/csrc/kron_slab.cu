@@ -49,6 +49,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include "kron_fibre.cuh"
 #include "kron_launch.h"
 #include "kron_ptx.cuh"
 
@@ -101,107 +102,6 @@ struct SlabShape
 
 constexpr int FLAG_X_TMA = 1; // slab arrived by bulk copy
 constexpr int FLAG_A_TMA = 2; // A_1..A_6 arrived by bulk copy (contiguous)
-
-// factor A (column major, A(i, j) at i + j N) into registers
-template <typename T, int N>
-__device__ __forceinline__ void load_factor(const T *A, T (&a)[N][N])
-{
-#pragma unroll
-  for (int j = 0; j < N; j++)
-  {
-    if constexpr (sizeof(T) == 8 && N % 2 == 0)
-    {
-#pragma unroll
-      for (int i = 0; i < N; i += 2)
-      {
-        const double2 u = *reinterpret_cast<const double2 *>(A + i + j * N);
-        a[i][j]         = u.x;
-        a[i + 1][j]     = u.y;
-      }
-    }
-    else if constexpr (sizeof(T) == 4 && N % 2 == 0)
-    {
-#pragma unroll
-      for (int i = 0; i < N; i += 2)
-      {
-        const float2 u = *reinterpret_cast<const float2 *>(A + i + j * N);
-        a[i][j]        = u.x;
-        a[i + 1][j]    = u.y;
-      }
-    }
-    else
-    {
-#pragma unroll
-      for (int i = 0; i < N; i++)
-        a[i][j] = A[i + j * N];
-    }
-  }
-}
-
-// v is an n x n block, v[a N + b]: apply_fast applies A along b (the faster
-// mode), apply_slow along a
-template <typename T, int N>
-__device__ __forceinline__ void apply_fast(T (&v)[N * N], const T *A)
-{
-  T a[N][N];
-  load_factor<T, N>(A, a);
-#pragma unroll
-  for (int r = 0; r < N; r++)
-  {
-    T t[N];
-#pragma unroll
-    for (int i = 0; i < N; i++)
-    {
-      T z = a[i][0] * v[r * N];
-#pragma unroll
-      for (int j = 1; j < N; j++)
-        z = fma(a[i][j], v[r * N + j], z);
-      t[i] = z;
-    }
-#pragma unroll
-    for (int i = 0; i < N; i++)
-      v[r * N + i] = t[i];
-  }
-}
-
-template <typename T, int N>
-__device__ __forceinline__ void apply_slow(T (&v)[N * N], const T *A, int rot = 0)
-{
-  T a[N][N];
-  if (rot == 0)
-    load_factor<T, N>(A, a);
-  else
-  {
-    // rows of v hold rows (r + rot) mod N: the factor with rows and columns
-    // rotated the same way gives the rotated rows of the product
-#pragma unroll
-    for (int i = 0; i < N; i++)
-#pragma unroll
-      for (int j = 0; j < N; j++)
-      {
-        const int ri = i + rot < N ? i + rot : i + rot - N;
-        const int rj = j + rot < N ? j + rot : j + rot - N;
-        a[i][j]      = A[ri + rj * N];
-      }
-  }
-#pragma unroll
-  for (int c = 0; c < N; c++)
-  {
-    T t[N];
-#pragma unroll
-    for (int i = 0; i < N; i++)
-    {
-      T z = a[i][0] * v[c];
-#pragma unroll
-      for (int j = 1; j < N; j++)
-        z = fma(a[i][j], v[j * N + c], z);
-      t[i] = z;
-    }
-#pragma unroll
-    for (int i = 0; i < N; i++)
-      v[i * N + c] = t[i];
-  }
-}
 
 // pass A: modes 5 (A_5, slow) and 6 (A_6, fast) on the contiguous fibre f.
 // FP64 fibres of n^2 = 36 elements start 18 16-byte units apart, so lanes f

@@ -195,7 +195,8 @@ extern "C" int kron_autotune(int d, int n, int precision, int batch, int *varian
   // per block, the cluster kernel at cluster sizes 1, 2, 4 (FP64 n = 8: on
   // the tensor cores and on CUDA cores; FP64 n = 6: W in the workspace or
   // on chip)
-  std::vector<std::pair<int, int>> cand = {{VAR_MMA8, 0}, {VAR_PIPE, 0}, {VAR_SLAB, 0}};
+  std::vector<std::pair<int, int>> cand = {
+      {VAR_MMA8, 0}, {VAR_PIPE, 0}, {VAR_SLAB, KRON_SLAB_RESIDENT}, {VAR_SLAB, 0}};
   const int ngmax = sq_entries_max(precision, d, n, false);
   for (int ng = 1; ng <= ngmax; ng *= 2)
     cand.push_back({VAR_SQ, ng});
