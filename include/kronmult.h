@@ -370,7 +370,11 @@ int kron_l2_persist_reset(kron_stream_t stream);
  *                       (FP64 d = 6, n = 6; that form also runs, without
  *                       the bit, when the caller passes no W), plus
  *                       KRON_BIG_NO_L2_HINTS to drop the L2 cache policies
- *                       that keep W resident (a comparison form)
+ *                       that keep W resident (a comparison form), or
+ *                       KRON_BIG_RING for the ring form (d = 6, n = 6..8,
+ *                       FP64 and FP32): both phases from one queue through
+ *                       a ring of W vectors (the built-in choice for large
+ *                       enough batches with a workspace)
  *   KRON_VARIANT_LARGE  two-phase launches through the workspace W
  *   KRON_VARIANT_SPLIT_TC  split precision (KRON_PREC_SPLIT) for d = 6,
  *                       n = 8 in the batched layout with W: the two phases'
@@ -422,6 +426,7 @@ int kron_l2_persist_reset(kron_stream_t stream);
 #define KRON_VARIANT_SPLIT_TC 8
 #define KRON_BIG_CUDA_CORES 256
 #define KRON_BIG_SMEM_W 512
+#define KRON_BIG_RING 2048
 #define KRON_BIG_NO_L2_HINTS 1024
 #define KRON_SLAB_NO_ROTATE 1
 #define KRON_SLAB_WHOLE 2

@@ -248,6 +248,8 @@ BIG_CUDA_CORES = 256
 BIG_SMEM_W = 512
 # "big" param bit: no L2 cache policies on W, x and y (comparison form)
 BIG_NO_L2_HINTS = 1024
+# "big" param bit: the ring form (both phases from one queue, d = 6, n = 6..8)
+BIG_RING = 2048
 # "slab" param bit: no lane rotation in the first FP64 pass (comparison form)
 SLAB_NO_ROTATE = 1
 # "slab" param bit: clusters of 6 blocks holding whole slabs (comparison form)

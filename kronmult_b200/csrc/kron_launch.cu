@@ -610,8 +610,12 @@ int launch_variant(Params p, int prec, const Workspace &ws, int variant, int par
     return KRON_ERROR_NOT_SUPPORTED;
   }
   case VAR_BIG:
+    if (param & KRON_BIG_RING)
+      return launch_variant(p, prec, ws, VAR_RING, 0, stream);
     return big_supported(p, prec) ? launch_big(p, ws, prec, param, stream)
                                   : KRON_ERROR_NOT_SUPPORTED;
+  case VAR_RING:
+    return ring_supported(p, prec) ? launch_ring(p, prec, ws, stream) : KRON_ERROR_NOT_SUPPORTED;
   case VAR_RESIDENT:
     return resident_supported(p, prec) ? launch_resident(p, stream)
                                        : KRON_ERROR_NOT_SUPPORTED;
@@ -636,6 +640,14 @@ int launch_variant(Params p, int prec, const Workspace &ws, int variant, int par
 // 481 against 13.6 / 20.8 / 27.0 / 938.
 static bool prefer_resident(const Params &p) { return p.eend - p.ebase >= 40; }
 
+// FP64 d = 6, n = 6: the ring's two phases are a serial chain of about 40 us,
+// a cluster of twelve an entry (slab) finishes 21 entries in 14 us;
+// microseconds at 80 / 160 / 320 / 4096 entries: 54 / 71 / 115 / 1204
+// against 39 / 70 / 132 / 1428.  n = 7, 8: the cluster two-phase kernel is
+// slower at every batch (3 entries, FP64: 136 against 44 us and 121 against
+// 60 us).
+static bool prefer_ring(const Params &p) { return p.n[0] > 6 || p.eend - p.ebase >= 160; }
+
 int launch_kron(Params p, int prec, const Workspace &ws, cudaStream_t stream)
 {
   if (p.batch <= 0 || p.eend <= p.ebase)
@@ -657,22 +669,25 @@ int launch_kron(Params p, int prec, const Workspace &ws, cudaStream_t stream)
   // default order: the specialised kernels, then the general ones
   // (VAR_SPLIT_TC: split precision at d = 6, n = 8 on the tcgen05 tensor
   // cores, 3.6 ms for 256 entries against 7.5 ms for the CUDA-core split)
-  // (VAR_RESIDENT: from the batch on that fills the GPU, see prefer_resident)
-  static const int order[] = {VAR_MMA8, VAR_PIPE, VAR_RESIDENT, VAR_SLAB, VAR_SQ,
+  // (VAR_RESIDENT and VAR_RING: from the batch on that fills the GPU, see
+  // prefer_resident and prefer_ring; a ring without the workspace for it
+  // leaves the call to the next form)
+  static const int order[] = {VAR_MMA8, VAR_PIPE, VAR_RESIDENT, VAR_RING, VAR_SLAB, VAR_SQ,
                               VAR_GEN,  VAR_BIG,  VAR_SPLIT_TC, VAR_LARGE};
   for (int v : order)
   {
-    if (v == VAR_RESIDENT && !prefer_resident(p))
+    if ((v == VAR_RESIDENT && !prefer_resident(p)) || (v == VAR_RING && !prefer_ring(p)))
       continue;
     if ((v == VAR_MMA8 && std::getenv("KRON_DISABLE_MMA8")) ||
         (v == VAR_PIPE && std::getenv("KRON_DISABLE_PIPE")) ||
         (v == VAR_RESIDENT && std::getenv("KRON_DISABLE_RESIDENT")) ||
+        (v == VAR_RING && std::getenv("KRON_DISABLE_RING")) ||
         (v == VAR_SLAB && std::getenv("KRON_DISABLE_SLAB")) ||
         (v == VAR_BIG && std::getenv("KRON_DISABLE_BIG")) ||
         (v == VAR_SPLIT_TC && std::getenv("KRON_DISABLE_SPLIT_TC")))
       continue;
     const int rc = launch_variant(p, prec, ws, v, 0, stream);
-    if (rc != KRON_ERROR_NOT_SUPPORTED)
+    if (rc != KRON_ERROR_NOT_SUPPORTED && !(v == VAR_RING && rc == KRON_ERROR_WORKSPACE))
       return rc;
   }
   return KRON_ERROR_NOT_SUPPORTED;

@@ -63,6 +63,11 @@ int launch_big(Params p, const Workspace &ws, int prec, int cluster, cudaStream_
 bool resident_supported(const Params &p, int prec);
 int launch_resident(const Params &p, cudaStream_t stream);
 
+// Ring kernel for square d = 6 vectors beyond shared memory (n = 6..8) with a
+// workspace (kron_ring.cu).
+bool ring_supported(const Params &p, int prec);
+int launch_ring(const Params &p, int prec, const Workspace &ws, cudaStream_t stream);
+
 // Split precision (FP64 data, exact BF16 slice products on the tcgen05 tensor
 // cores) for square d = 6, n = 8 in the batched layout with a workspace W
 // (kron_splittc.cu).
@@ -81,11 +86,14 @@ enum Variant : int
   VAR_BIG   = 5, // cluster two-phase kernel; param = cluster size (0: default)
                  // | KRON_BIG_CUDA_CORES (FP64 n = 8 without tensor cores)
                  // | KRON_BIG_SMEM_W (FP64 n = 6: W in the cluster's shared memory)
+                 // | KRON_BIG_RING (VAR_RING)
   VAR_LARGE = 6, // two-phase launches through the workspace (param unused)
   VAR_SLAB  = 7, // slab-cluster kernel, no workspace; param: KRON_SLAB_NO_ROTATE
   VAR_SPLIT_TC = 8, // split precision d = 6, n = 8 on the tcgen05 tensor cores
   VAR_RESIDENT = 10, // FP32 vector resident in one block; in the tuning table it is
                     // VAR_SLAB with KRON_SLAB_RESIDENT
+  VAR_RING = 9,     // two-phase queue through a ring of W vectors; in the tuning table
+                    // it is VAR_BIG with KRON_BIG_RING
 };
 
 // Work items of a launch (launch_kron does this before any variant).

@@ -207,6 +207,7 @@ extern "C" int kron_autotune(int d, int n, int precision, int batch, int *varian
   // (fixed cluster of 2)
   if (precision == PREC_F64 && d == 6 && n == 6)
     cand.push_back({VAR_BIG, KRON_BIG_SMEM_W});
+  cand.push_back({VAR_BIG, KRON_BIG_RING});
   for (int cs : {1, 2, 4})
   {
     cand.push_back({VAR_BIG, cs});
