@@ -154,6 +154,40 @@ __device__ __forceinline__ int entry_index(const Params &p, int e)
   return p.perm ? p.perm[e] : e;
 }
 
+// Balanced contiguous range of positions for group gw of nw (warps, thread
+// groups): positions are split evenly; with output groups (seg_off) the split
+// points snap to the next group start, so that an output group is never
+// shared.
+__device__ __forceinline__ int snap_to_group(const Params &p, long long pos)
+{
+  int lo = p.ibase, hi = p.ibase + p.nitems; // first s with seg_off[s] >= pos
+  while (lo < hi)
+  {
+    const int mid = (lo + hi) >> 1;
+    if (p.seg_off[mid] < pos)
+      lo = mid + 1;
+    else
+      hi = mid;
+  }
+  return p.seg_off[lo];
+}
+
+__device__ __forceinline__ void group_range(const Params &p, int gw, int nw, int &eb, int &ee)
+{
+  if (p.seg_off)
+  {
+    const long long b = p.seg_off[p.ibase], tot = p.seg_off[p.ibase + p.nitems] - b;
+    eb = snap_to_group(p, b + tot * gw / nw);
+    ee = snap_to_group(p, b + tot * (gw + 1) / nw);
+  }
+  else
+  {
+    const long long tot = p.eend - p.ebase;
+    eb = p.ebase + (int)(tot * gw / nw);
+    ee = p.ebase + (int)(tot * (gw + 1) / nw);
+  }
+}
+
 // Barrier over one thread group of `nthreads` (a multiple of 32) with a
 // group-private id (1..15); the whole block uses __syncthreads().
 __device__ __forceinline__ void group_sync(int gid, int nthreads)

@@ -2,7 +2,8 @@
 //
 //  * square n in 2..8 whose n^d vector (and merge buffer) fits a block's
 //    shared memory            -> kron_sq_kernel<T, d, n>   (compile-time shape)
-//  * any other shape that fits -> kron_gen_kernel<T>        (runtime shape)
+//  * any other shape that fits -> kron_rect_kernel (FP64) or kron_gen_kernel<T>
+//    (runtime shape)
 //  * vectors too large for shared memory -> two launches of kron_gen_kernel
 //    through the caller's workspace W: phase 1 applies the trailing modes to
 //    every contiguous block of x (writing W), phase 2 applies the leading
@@ -279,8 +280,11 @@ static void setup_items(Params &p, const Workspace &ws)
   }
   if (p.accum == ACC_ATOMIC)
   {
-    // short runs of consecutive entries per item so equal outputs merge
-    p.chunk = 8;
+    // short runs of consecutive entries per item so equal outputs merge, as
+    // long as that leaves sixteen items an SM: a run is worked through in
+    // series (square d = 4, n = 7 on a grid of 400 elements with 9 couplings:
+    // 92.7 us in runs of 3, 85.6 us in runs of 1; n = 4: 16.7 and 14.1 us)
+    p.chunk = std::max(1, std::min(8, (p.eend - p.ebase) / (16 * device_info().sms)));
   }
   else
     p.chunk = 1;
@@ -601,6 +605,8 @@ int launch_variant(Params p, int prec, const Workspace &ws, int variant, int par
     void *args[]    = {&p};
     return launch_blocks(ki.fn, p.nitems, ng, block, smem, args, stream);
   }
+  case VAR_RECT:
+    return rect_supported(p, prec) ? launch_rect(p, stream) : KRON_ERROR_NOT_SUPPORTED;
   case VAR_GEN: {
     GenView v;
     if (gen_whole_view(p.d, p.m, p.n, merge, esize, v))
@@ -673,13 +679,14 @@ int launch_kron(Params p, int prec, const Workspace &ws, cudaStream_t stream)
   // prefer_resident and prefer_ring; a ring without the workspace for it
   // leaves the call to the next form)
   static const int order[] = {VAR_MMA8, VAR_PIPE, VAR_RESIDENT, VAR_RING, VAR_SLAB, VAR_SQ,
-                              VAR_GEN,  VAR_BIG,  VAR_SPLIT_TC, VAR_LARGE};
+                              VAR_RECT, VAR_GEN,  VAR_BIG,  VAR_SPLIT_TC, VAR_LARGE};
   for (int v : order)
   {
     if ((v == VAR_RESIDENT && !prefer_resident(p)) || (v == VAR_RING && !prefer_ring(p)))
       continue;
     if ((v == VAR_MMA8 && std::getenv("KRON_DISABLE_MMA8")) ||
         (v == VAR_PIPE && std::getenv("KRON_DISABLE_PIPE")) ||
+        (v == VAR_RECT && std::getenv("KRON_DISABLE_RECT")) ||
         (v == VAR_RESIDENT && std::getenv("KRON_DISABLE_RESIDENT")) ||
         (v == VAR_RING && std::getenv("KRON_DISABLE_RING")) ||
         (v == VAR_SLAB && std::getenv("KRON_DISABLE_SLAB")) ||

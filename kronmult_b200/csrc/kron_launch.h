@@ -29,6 +29,11 @@ bool plan_large(int d, const int *m, const int *n, int esize, bool merge, LargeP
 bool mma8_supported(const Params &p, int prec);
 int launch_mma8(Params p, cudaStream_t stream);
 
+// Runtime-shape kernel for whole FP64 vectors in shared memory, one shape a
+// launch (kron_rect.cu).
+bool rect_supported(const Params &p, int prec);
+int launch_rect(const Params &p, cudaStream_t stream);
+
 // TMA-pipelined register-blocked kernel for square n in {2..5}, 4-64 KB
 // vectors (kron_pipe.cu).
 bool pipe_supported(const Params &p, int prec);
@@ -90,6 +95,8 @@ enum Variant : int
   VAR_LARGE = 6, // two-phase launches through the workspace (param unused)
   VAR_SLAB  = 7, // slab-cluster kernel, no workspace; param: KRON_SLAB_NO_ROTATE
   VAR_SPLIT_TC = 8, // split precision d = 6, n = 8 on the tcgen05 tensor cores
+  VAR_RECT = 12,    // runtime-shape kernel for whole FP64 vectors (the built-in choice
+                    // where VAR_GEN's whole-vector form would run)
   VAR_RESIDENT = 10, // FP32 vector resident in one block; in the tuning table it is
                     // VAR_SLAB with KRON_SLAB_RESIDENT
   VAR_RING = 9,     // two-phase queue through a ring of W vectors; in the tuning table

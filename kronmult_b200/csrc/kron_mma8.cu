@@ -96,39 +96,6 @@ __device__ __forceinline__ void flush_acc(double (&acc)[8][2], double *y, int g,
     }
 }
 
-// Balanced contiguous range of positions for warp gw of nw: positions are
-// split evenly; with output groups (seg_off) the split points snap to the
-// next group start so a group is never shared between warps.
-__device__ __forceinline__ int snap_to_group(const Params &p, long long pos)
-{
-  int lo = p.ibase, hi = p.ibase + p.nitems; // first s with seg_off[s] >= pos
-  while (lo < hi)
-  {
-    const int mid = (lo + hi) >> 1;
-    if (p.seg_off[mid] < pos)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  return p.seg_off[lo];
-}
-
-__device__ __forceinline__ void warp_range(const Params &p, int gw, int nw, int &eb, int &ee)
-{
-  if (p.seg_off)
-  {
-    const long long b = p.seg_off[p.ibase], tot = p.seg_off[p.ibase + p.nitems] - b;
-    eb = snap_to_group(p, b + tot * gw / nw);
-    ee = snap_to_group(p, b + tot * (gw + 1) / nw);
-  }
-  else
-  {
-    const long long tot = p.eend - p.ebase;
-    eb = p.ebase + (int)(tot * gw / nw);
-    ee = p.ebase + (int)(tot * (gw + 1) / nw);
-  }
-}
-
 __global__ void __launch_bounds__(WARPS * 32) kron_n8d3_mma_kernel(const __grid_constant__ Params p)
 {
   extern __shared__ __align__(16) double smem[];
@@ -139,7 +106,7 @@ __global__ void __launch_bounds__(WARPS * 32) kron_n8d3_mma_kernel(const __grid_
   double *xbase = smem + warp * WARP_SMEM;
 
   int eb, ee;
-  warp_range(p, blockIdx.x * WARPS + warp, gridDim.x * WARPS, eb, ee);
+  group_range(p, blockIdx.x * WARPS + warp, gridDim.x * WARPS, eb, ee);
   if (eb >= ee)
     return;
   int e = eb; // position being computed; e+1 has operands in flight, e+2 pointers

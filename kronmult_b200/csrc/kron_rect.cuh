@@ -1,0 +1,143 @@
+// Mode products of runtime (rectangular) shapes, prepared on the host.
+//
+// A vector's mode products run as a list of steps, each out of place on
+// fibres of one mode: fibre f = (o, r), o = f / inner, reads
+// cur[(o nq + j) inner + r] and writes nxt[(o mq + i) inner + r].  The list
+// is computed once (per launch or per plan), so that a thread's work per step
+// is its fibres only: no shapes to multiply out, and o by a multiplication.
+// The factors lie in shared memory in the order of the steps.
+#pragma once
+
+#include "kron_internal.cuh"
+
+namespace kron {
+
+struct RectStep
+{
+  int inner;          // elements between consecutive indices of the mode
+  int nfib;           // fibres (of one row, where the buffer holds several)
+  unsigned magic;     // ceil(2^32 / inner), 0 for inner = 1
+  unsigned char nq, mq, mode, pad;
+};
+static_assert(sizeof(RectStep) == 16, "read as one 16-byte word");
+
+// Steps of the modes [mode0, mode0 + dd) in the given order; C columns ride
+// along as the fastest index.  Exact while the elements of a buffer times the
+// largest inner stay below 2^32 (buffers fit shared memory).
+inline void rect_plan(RectStep *st, int dd, const int *m, const int *n, int mode0, bool forward,
+                      int C)
+{
+  int dims[MAXD];
+  for (int q = 0; q < dd; q++)
+    dims[q] = n[q];
+  for (int s = 0; s < dd; s++)
+  {
+    const int q = forward ? s : dd - 1 - s;
+    long long outer = 1, inner = C;
+    for (int u = 0; u < q; u++)
+      outer *= dims[u];
+    for (int u = q + 1; u < dd; u++)
+      inner *= dims[u];
+    st[s].inner = (int)inner;
+    st[s].nfib  = (int)(outer * inner);
+    st[s].magic = inner == 1 ? 0u : (unsigned)(((1ULL << 32) + inner - 1) / inner);
+    st[s].nq    = (unsigned char)n[q];
+    st[s].mq    = (unsigned char)m[q];
+    st[s].mode  = (unsigned char)(mode0 + q);
+    st[s].pad   = 0;
+    dims[q]     = m[q];
+  }
+}
+
+// Factors of up to AREG_MAX elements are held in registers, larger ones are read
+// from shared memory at every use.
+template <typename T, int AREG_MAX, int NQ, int MQ>
+__device__ __forceinline__ void rect_fibres(const T *cur, T *nxt, const T *A, int inner,
+                                            unsigned magic, int nfib, int t, int GS)
+{
+  constexpr bool AREG = NQ * MQ <= AREG_MAX;
+  T a[AREG ? MQ : 1][AREG ? NQ : 1];
+  if constexpr (AREG)
+  {
+    if (t < nfib)
+#pragma unroll
+      for (int j = 0; j < NQ; j++)
+#pragma unroll
+        for (int i = 0; i < MQ; i++)
+          a[i][j] = A[i + j * MQ];
+  }
+  for (int f = t; f < nfib; f += GS)
+  {
+    const int o  = magic ? (int)__umulhi((unsigned)f, magic) : f;
+    const int oi = o * inner;
+    const T *src = cur + f + oi * (NQ - 1);
+    T *dst       = nxt + f + oi * (MQ - 1);
+    T x[NQ];
+#pragma unroll
+    for (int j = 0; j < NQ; j++)
+      x[j] = src[j * inner];
+#pragma unroll
+    for (int i = 0; i < MQ; i++)
+    {
+      T z = T(0);
+#pragma unroll
+      for (int j = 0; j < NQ; j++)
+        z = fma(AREG ? a[AREG ? i : 0][AREG ? j : 0] : A[i + j * MQ], x[j], z);
+      dst[i * inner] = z;
+    }
+  }
+}
+
+// Sizes beyond 8: one output element at a time (rare shapes, kept simple).
+template <typename T>
+__device__ __noinline__ void rect_step_any(const T *cur, T *nxt, const T *A, int nq, int mq,
+                                           int inner, unsigned magic, int nfib, int t, int GS)
+{
+  for (int f = t; f < nfib; f += GS)
+  {
+    const int o  = magic ? (int)__umulhi((unsigned)f, magic) : f;
+    const T *src = cur + f + o * inner * (nq - 1);
+    T *dst       = nxt + f + o * inner * (mq - 1);
+    for (int i = 0; i < mq; i++)
+    {
+      T z = T(0);
+      for (int j = 0; j < nq; j++)
+        z = fma(A[i + j * mq], src[j * inner], z);
+      dst[i * inner] = z;
+    }
+  }
+}
+
+// all steps over `rows` consecutive vectors; cur holds the result at the end
+template <typename T, int AREG_MAX>
+__device__ __forceinline__ void rect_modes(const RectStep *st, int ns, int rows, T *&cur, T *&nxt,
+                                           const T *As, int t, int GS, int g)
+{
+  for (int s = 0; s < ns; s++)
+  {
+    const RectStep q = st[s];
+    const int nfib   = q.nfib * rows, inner = q.inner;
+    switch (q.nq <= 8 && q.mq <= 8 ? q.nq * 16 + q.mq : 0)
+    {
+#define KRON_RM(NQ_, MQ_)                                                                       \
+  case NQ_ * 16 + MQ_:                                                                          \
+    rect_fibres<T, AREG_MAX, NQ_, MQ_>(cur, nxt, As, inner, q.magic, nfib, t, GS);                        \
+    break;
+#define KRON_RM_ROW(NQ_)                                                                        \
+  KRON_RM(NQ_, 1) KRON_RM(NQ_, 2) KRON_RM(NQ_, 3) KRON_RM(NQ_, 4) KRON_RM(NQ_, 5)              \
+  KRON_RM(NQ_, 6) KRON_RM(NQ_, 7) KRON_RM(NQ_, 8)
+      KRON_RM_ROW(1) KRON_RM_ROW(2) KRON_RM_ROW(3) KRON_RM_ROW(4)
+      KRON_RM_ROW(5) KRON_RM_ROW(6) KRON_RM_ROW(7) KRON_RM_ROW(8)
+#undef KRON_RM_ROW
+#undef KRON_RM
+    default: rect_step_any(cur, nxt, As, q.nq, q.mq, inner, q.magic, nfib, t, GS); break;
+    }
+    As += q.nq * q.mq;
+    T *tmp = cur;
+    cur    = nxt;
+    nxt    = tmp;
+    group_sync(g, GS);
+  }
+}
+
+} // namespace kron
