@@ -24,7 +24,16 @@
 // kron_vplan_execute_async runs one persistent kernel: the huge queue, then
 // the block, half, quad and warp classes, each from its own device work
 // counter.  All operands reach shared memory by cp.async, so a block keeps
-// every byte of its current item in flight at once.  On a non-default
+// every byte of its current item in flight at once.  The mode products follow
+// a list of steps that the plan computed for each entry (kron_rect.cuh); it
+// arrives with the next item's descriptor.
+//
+// 20000 entries with d in 1..6 and sizes from {2, 3, 4, 6, 8} (0.99 GB): 0.552
+// ms, against 0.921 ms when every thread worked out each step's shape and
+// divided per fibre (the products were 17 of 29 thousand cycles of a chunk
+// item).  Two blocks of 256 threads with factors of up to 36 elements in
+// registers are the best split: three blocks (80 registers) 0.616, two of 512
+// threads 0.827, one of 512 threads 0.600 ms.  On a non-default
 // stream the counter reset and the launch are captured once into a CUDA
 // graph and replayed while the operand arrays stay the same.
 #include <algorithm>
@@ -35,6 +44,7 @@
 
 #include "kron_launch.h"
 #include "kron_ptx.cuh"
+#include "kron_rect.cuh"
 
 using namespace kron;
 
@@ -42,6 +52,7 @@ namespace {
 
 constexpr int VP_THREADS = 256;
 constexpr int VP_WARPS   = VP_THREADS / 32;
+constexpr int VP_AREG    = 36;    // elements of a factor held in registers
 constexpr int VP_MINB    = 2;     // blocks per SM the shared-memory budget leaves room for
 constexpr int WARP_MAX   = 512;   // elements of the largest intermediate, warp class
 constexpr int CLS_WARP = 0, CLS_QUAD = 1, CLS_HALF = 2, CLS_BLOCK = 3, CLS_HUGE = 4;
@@ -53,17 +64,26 @@ struct VDesc
   // fetched as twelve 32-bit words by the kernel's fetch stages
   long long woff;       // huge: element offset of the entry's workspace region
   int k;                // entry index (operands at pA[6k + l], pX[k], pY[k])
-  unsigned char d, fwd, q, C;  // order; huge: head modes q, tile columns C
-  unsigned char m[6], n[6];
+  unsigned char d, q, C, pad;  // modes; huge: head modes q, tile columns C
+  int nin, nout;        // elements of x and y (huge: of one tail row)
+  int hin, hout;        // huge: head rows in and out
   int mi;               // buffer elements: the largest intermediate of the chosen
-                        // order (huge: of one chunk of R head rows)
+                        // order (huge: of one chunk of R head rows), and two so
+                        // that x may start at an odd element
   int mi2;              // huge: phase-2 buffer elements (tile rows x C)
-  unsigned char fwd1, fwd2;   // huge: order of the tail / head modes
-  unsigned short R;           // huge: head rows per chunk item
-  int nchunk;                 // huge: chunk items (its tile items wait for all)
+  int R;                // huge: head rows per chunk item
+  int nchunk;           // huge: chunk items (its tile items wait for all)
 };
 
 static_assert(sizeof(VDesc) == 48, "VDesc is fetched as 12 words");
+
+// an entry's mode products (huge: the d - q tail steps, then the q head steps)
+struct VSteps
+{
+  RectStep st[MAXD];
+};
+constexpr int VSTEP_WORDS = sizeof(VSteps) / 4;
+static_assert(VSTEP_WORDS <= 32, "fetched as a word a lane");
 
 // kind 0: chunk item, head rows [lo, hi); kind 1: tile item, column tile lo
 // of the huge entry desc[e]
@@ -75,6 +95,7 @@ struct VItem
 struct VParams
 {
   const VDesc *desc;          // [huge | block | half | quad | warp]
+  const VSteps *steps;        // the same order
   const VItem *items;         // the huge queue
   int nhuge, nblock, nhalf, nquad, nwarp;
   int nitems;
@@ -107,85 +128,119 @@ __device__ __forceinline__ int ld_acquire(const int *p)
   return v;
 }
 
-// The view's factors (leading dimension m_l: each contiguous) into As.
-__device__ __forceinline__ void vp_load_factors(const GenView &v, double *As,
+// The steps' factors (leading dimension m_l: each contiguous) into As in step
+// order, a warp a step.
+__device__ __forceinline__ void vp_load_factors(const RectStep *st, int ns, double *As,
                                                 const double *const *A, int t, int GS)
 {
+  const int warp = t >> 5, lane = t & 31, nw = GS >> 5;
   int o = 0;
-  for (int q = 0; q < v.dd; q++)
+  for (int s = 0; s < ns; s++)
   {
-    const int sz    = v.mm[q] * v.nn[q];
-    const double *a = A[v.mode0 + q];
-    for (int u = t; u < sz; u += GS)
-      cp8(As + o + u, a + u);
+    const int sz = st[s].nq * st[s].mq;
+    if (s % nw == warp)
+    {
+      const double *a = A[st[s].mode];
+      for (int u = lane; u < sz; u += 32)
+        cp8(As + o + u, a + u);
+    }
     o += sz;
   }
 }
 
-// rows consecutive vectors of the view (x contiguous) computed by a group
-// of GS threads in buffers b0 / b1 (each >= rows x the largest
-// intermediate), factors at As; the results go to out (contiguous).
-// hook(s) runs the next item's fetch stage s at four points: after the
-// copies are issued, after they land, before the results go out, and
-// before the closing barrier.
-template <typename Hook>
-__device__ __forceinline__ void vp_run(const GenView &v, int rows, const double *x, double *out,
-                                       int accum, double *b0, double *b1, double *As,
-                                       const double *const *A, int t, int GS, int g,
+// `count` elements at src to buf + the offset src has in its 16-byte unit,
+// 16 bytes at a time but for the ends; returns where they start.
+__device__ __forceinline__ double *vp_load_x(double *buf, const double *src, int count, int t,
+                                             int GS)
+{
+  const int sh = (int)((reinterpret_cast<uintptr_t>(src) >> 3) & 1);
+  const int u1 = (sh + count) / 2; // units [sh, u1) lie whole in the source
+  for (int u = sh + t; u < u1; u += GS)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ptx::smem_addr(buf + 2 * u)),
+                 "l"(src - sh + 2 * u)
+                 : "memory");
+  if (sh && t == 0)
+    cp8(buf + 1, src);
+  if (((sh + count) & 1) && t == GS - 1)
+    cp8(buf + sh + count - 1, src + count - 1);
+  return buf + sh;
+}
+
+// rows consecutive vectors (x contiguous) computed by a group of GS threads
+// in buffers b0 / b1 (each >= rows x the largest intermediate and two),
+// factors at As; the results go to out (contiguous): added into y, or stored
+// into the workspace region.  hook(s) runs the next item's fetch stage s at
+// four points: after the copies are issued, after they land, before the
+// results go out, and before the closing barrier.
+template <bool STORE, typename Hook>
+__device__ __forceinline__ void vp_run(const RectStep *st, int ns, int rows, int nin, int nout,
+                                       const double *x, double *out, double *b0, double *b1,
+                                       double *As, const double *const *A, int t, int GS, int g,
                                        const Hook &hook)
 {
-  vp_load_factors(v, As, A, t, GS);
-  int rin = rows, rout = rows;
-  for (int q = 0; q < v.dd; q++)
-  {
-    rin *= v.nn[q];
-    rout *= v.mm[q];
-  }
-  for (int i = t; i < rin; i += GS)
-    cp8(b0 + i, x + i);
+  vp_load_factors(st, ns, As, A, t, GS);
+  double *cur = vp_load_x(b0, x, rows * nin, t, GS), *nxt = b1;
   hook(1);
   cp_wait_all();
   group_sync(g, GS);
   hook(2);
-  double *cur = b0, *nxt = b1;
-  gen_apply_modes<double, PREC_F64, true>(v, cur, nxt, As, 1, t, GS, g, rows);
+  rect_modes<double, VP_AREG>(st, ns, rows, cur, nxt, As, t, GS, g);
   hook(3);
-  group_flush(accum, out, cur, cur, false, rout, t, GS);
+  const int count = rows * nout;
+  if constexpr (STORE)
+  {
+    if (ptx::aligned16(cur) && ptx::aligned16(out))
+    {
+      for (int i = t; i < count / 2; i += GS)
+        reinterpret_cast<double2 *>(out)[i] = reinterpret_cast<const double2 *>(cur)[i];
+      if ((count & 1) && t == 0)
+        out[count - 1] = cur[count - 1];
+    }
+    else
+      for (int i = t; i < count; i += GS)
+        out[i] = cur[i];
+  }
+  else
+    for (int i = t; i < count; i += GS)
+      red_add(out + i, cur[i]);
   hook(4);
   group_sync(g, GS);
 }
 
-// One column tile of a huge entry's region: rows of C columns at stride
+// One column tile of a huge entry's region: rin rows of C columns at stride
 // in_row (the first Cc valid, the rest zero-filled), the head modes, and
-// the Cc valid columns added into y (row stride out_row).  Whole block;
-// hook as for vp_run.
+// the Cc valid columns added into y (rout rows, row stride out_row).  Whole
+// block; hook as for vp_run.
 template <typename Hook>
-__device__ __forceinline__ void vp_run_tile(const GenView &v, const double *w, long long in_row,
-                                            int C, int Cc, double *y, long long out_row,
-                                            double *b0, double *b1, double *As,
+__device__ __forceinline__ void vp_run_tile(const RectStep *st, int ns, int rin, int rout,
+                                            const double *w, int in_row, int C, int Cc, double *y,
+                                            int out_row, double *b0, double *b1, double *As,
                                             const double *const *A, int tid, const Hook &hook)
 {
-  vp_load_factors(v, As, A, tid, VP_THREADS);
-  int rin = 1, rout = 1;
-  for (int q = 0; q < v.dd; q++)
-  {
-    rin *= v.nn[q];
-    rout *= v.mm[q];
-  }
+  vp_load_factors(st, ns, As, A, tid, VP_THREADS);
   const int lane = tid & 31, warp = tid >> 5;
-  for (int h = warp; h < rin; h += VP_WARPS)
-    for (int c = lane; c < C; c += 32)
-      cp8(b0 + h * C + c, w + h * in_row + (c < Cc ? c : 0), c < Cc);
+  if (((C | Cc | in_row) & 1) == 0 && ptx::aligned16(w))
+  {
+    for (int h = warp; h < rin; h += VP_WARPS)
+      for (int c = 2 * lane; c < C; c += 64)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(ptx::smem_addr(b0 + h * C + c)),
+                     "l"(w + (long long)h * in_row + (c < Cc ? c : 0)), "r"(c < Cc ? 16 : 0)
+                     : "memory");
+  }
+  else
+    for (int h = warp; h < rin; h += VP_WARPS)
+      for (int c = lane; c < C; c += 32)
+        cp8(b0 + h * C + c, w + (long long)h * in_row + (c < Cc ? c : 0), c < Cc);
   hook(1);
   cp_wait_all();
   __syncthreads();
   hook(2);
   double *cur = b0, *nxt = b1;
-  gen_apply_modes<double, PREC_F64, true>(v, cur, nxt, As, C, tid, VP_THREADS, 0);
+  rect_modes<double, VP_AREG>(st, ns, 1, cur, nxt, As, tid, VP_THREADS, 0);
   hook(3);
   for (int i = warp; i < rout; i += VP_WARPS)
     for (int c = lane; c < Cc; c += 32)
-      red_add(y + i * out_row + c, cur[i * C + c]);
+      red_add(y + (long long)i * out_row + c, cur[i * C + c]);
   hook(4);
   __syncthreads();
 }
@@ -200,6 +255,7 @@ struct NextSlot
   int ready;             // huge tile item: its entry's chunks were complete
   VItem it;              // huge queue only
   VDesc e;
+  VSteps s;
   const double *ptr[8];  // A_1..A_6, x, y
 };
 
@@ -207,6 +263,7 @@ struct NextSlot
 struct Fetch
 {
   int r;                 // lane 0: the counter's old value; lanes: a word in flight
+  int w;                 // lanes: a word of the steps in flight
   int nidx;
   const double *p;       // lanes 0-7: a pointer in flight
 };
@@ -236,6 +293,8 @@ __device__ __forceinline__ void fetch_stage(int s, Fetch &f, NextSlot &slot, con
         f.r = reinterpret_cast<const int *>(vp.items + f.nidx)[lane];
       if (!HUGE && lane < 12)
         f.r = reinterpret_cast<const int *>(list + f.nidx)[lane];
+      if (!HUGE && lane < VSTEP_WORDS)
+        f.w = reinterpret_cast<const int *>(vp.steps + (list - vp.desc) + f.nidx)[lane];
     }
     return;
   }
@@ -251,11 +310,15 @@ __device__ __forceinline__ void fetch_stage(int s, Fetch &f, NextSlot &slot, con
       __syncwarp();
       if (more && lane < 12)
         f.r = reinterpret_cast<const int *>(vp.desc + slot.it.e)[lane];
+      if (more && lane < VSTEP_WORDS)
+        f.w = reinterpret_cast<const int *>(vp.steps + slot.it.e)[lane];
     }
     else if (s == 3)
     {
       if (more && lane < 12)
         reinterpret_cast<int *>(&slot.e)[lane] = f.r;
+      if (more && lane < VSTEP_WORDS)
+        reinterpret_cast<int *>(&slot.s)[lane] = f.w;
       __syncwarp();
       if (more && lane < 8)
       {
@@ -282,6 +345,8 @@ __device__ __forceinline__ void fetch_stage(int s, Fetch &f, NextSlot &slot, con
         slot.idx = f.nidx;
       if (more && lane < 12)
         reinterpret_cast<int *>(&slot.e)[lane] = f.r;
+      if (more && lane < VSTEP_WORDS)
+        reinterpret_cast<int *>(&slot.s)[lane] = f.w;
       __syncwarp();
       if (more && lane < 8)
       {
@@ -296,41 +361,6 @@ __device__ __forceinline__ void fetch_stage(int s, Fetch &f, NextSlot &slot, con
         slot.ptr[lane] = f.p;
     }
   }
-}
-
-__device__ __forceinline__ void vp_view(GenView &v, const VDesc &e, int mode0, int dd)
-{
-  v.dd    = dd;
-  v.mode0 = mode0;
-  for (int q = 0; q < dd; q++)
-  {
-    v.mm[q] = e.m[mode0 + q];
-    v.nn[q] = e.n[mode0 + q];
-  }
-  v.forward = e.fwd;
-  v.C       = 1;
-  v.in_row = v.out_row = 1;
-  v.total_cols         = 1;
-}
-
-// Sizes of a huge entry's split: head inputs Nhead, tail inputs / outputs
-// Ntail, Mtail (phase 1 maps each head row of Ntail elements to Mtail).
-struct HugeDims
-{
-  int Nhead, Ntail, Mtail;
-};
-
-__device__ __forceinline__ HugeDims huge_dims(const VDesc &e)
-{
-  HugeDims h{1, 1, 1};
-  for (int l = 0; l < e.q; l++)
-    h.Nhead *= e.n[l];
-  for (int l = e.q; l < e.d; l++)
-  {
-    h.Ntail *= e.n[l];
-    h.Mtail *= e.m[l];
-  }
-  return h;
 }
 
 // Thread 0 polls the entry's chunk counter (acquire) until `need` chunk
@@ -362,54 +392,41 @@ __device__ __forceinline__ bool vp_wait_chunks(const VParams &vp, int e, int nee
   return *s_flag != 0;
 }
 
-// Read the slot into the item's registers (every thread of the group).
-__device__ __forceinline__ void slot_read(const NextSlot &slot, VDesc &e, const double *A[6],
-                                          const double *&x, double *&y)
-{
-  e = slot.e;
-  for (int l = 0; l < 6; l++)
-    A[l] = slot.ptr[l];
-  x = slot.ptr[6];
-  y = const_cast<double *>(slot.ptr[7]);
-}
-
 // Entries of one class run by groups of GS threads, VP_THREADS / GS per
-// block, each group with its own slice of shared memory, barrier and slot.
+// block, each group with its own slice of shared memory, barrier and slots
+// (the current item's and the next one's).
 template <int GS>
 __device__ __forceinline__ void group_class(const VParams &vp, const VDesc *list, int n,
-                                            int *counter, double *smem, NextSlot *slots, int tid)
+                                            int *counter, double *smem, NextSlot (*slots)[2],
+                                            int tid)
 {
   constexpr int NG = VP_THREADS / GS;
   const int g = tid / GS, t = tid - (tid / GS) * GS, lane = tid & 31;
-  double *b0     = smem + (long long)g * ((vp.budget / NG) & ~1);
-  NextSlot &slot = slots[g];
-  const bool fw  = t < 32; // the group's first warp fetches
-  Fetch f{0, 0, nullptr};
+  double *b0    = smem + (long long)g * ((vp.budget / NG) & ~1);
+  const bool fw = t < 32; // the group's first warp fetches
+  Fetch f{0, 0, 0, nullptr};
   if (fw)
     for (int st = 0; st < 4; st++)
     {
-      fetch_stage<false>(st, f, slot, vp, list, n, counter, lane);
+      fetch_stage<false>(st, f, slots[g][0], vp, list, n, counter, lane);
       __syncwarp();
     }
   group_sync(g, GS);
-  const double *A[6];
-  const double *x;
-  double *y;
-  VDesc e;
-  while (true)
+  for (int b = 0;; b ^= 1)
   {
-    const int idx = slot.idx;
-    if (idx >= n)
+    const NextSlot &slot = slots[g][b];
+    NextSlot &next       = slots[g][b ^ 1];
+    if (slot.idx >= n)
       break;
-    slot_read(slot, e, A, x, y);
     if (fw)
-      fetch_stage<false>(0, f, slot, vp, list, n, counter, lane);
-    GenView v;
-    vp_view(v, e, 0, e.d);
-    vp_run(v, 1, x, y, ACC_ATOMIC, b0, b0 + e.mi, b0 + 2 * e.mi, A, t, GS, g, [&](int st) {
-      if (fw && st < 4)
-        fetch_stage<false>(st, f, slot, vp, list, n, counter, lane);
-    });
+      fetch_stage<false>(0, f, next, vp, list, n, counter, lane);
+    const VDesc &e = slot.e;
+    vp_run<false>(slot.s.st, e.d, 1, e.nin, e.nout, slot.ptr[6],
+                  const_cast<double *>(slot.ptr[7]), b0, b0 + e.mi, b0 + 2 * e.mi, slot.ptr, t,
+                  GS, g, [&](int st) {
+                    if (fw && st < 4)
+                      fetch_stage<false>(st, f, next, vp, list, n, counter, lane);
+                  });
   }
   __syncthreads(); // the next class lays its slices (and slots) over these
 }
@@ -420,48 +437,39 @@ __global__ void __launch_bounds__(VP_THREADS, VP_MINB)
 {
   extern __shared__ __align__(16) double smem[];
   __shared__ int s_flag;
-  __shared__ NextSlot s_slot[VP_WARPS];
+  __shared__ NextSlot s_slot[VP_WARPS][2];
   const int tid = threadIdx.x, lane = tid & 31;
   const bool fw = tid < 32;
-  const double *A[6];
-  const double *x;
-  double *y;
-  VDesc e;
   bool dead = false; // a chunk wait of this block gave up: skip later tile items
 
-  NextSlot &slot = s_slot[0];
-  Fetch f{0, 0, nullptr};
+  Fetch f{0, 0, 0, nullptr};
   if (fw)
     for (int st = 0; st < 5; st++)
     {
-      fetch_stage<true>(st, f, slot, vp, nullptr, vp.nitems, &vp.counters[0], lane);
+      fetch_stage<true>(st, f, s_slot[0][0], vp, nullptr, vp.nitems, &vp.counters[0], lane);
       __syncwarp();
     }
   __syncthreads();
-  auto hook = [&](int st) {
-    if (fw)
-      fetch_stage<true>(st, f, slot, vp, nullptr, vp.nitems, &vp.counters[0], lane);
-  };
-  while (true)
+  for (int b = 0;; b ^= 1)
   {
+    const NextSlot &slot = s_slot[0][b];
+    NextSlot &next       = s_slot[0][b ^ 1];
     if (slot.idx >= vp.nitems)
       break;
-    const VItem it   = slot.it;
-    const bool ready = slot.ready != 0;
-    slot_read(slot, e, A, x, y);
-    if (fw)
-      fetch_stage<true>(0, f, slot, vp, nullptr, vp.nitems, &vp.counters[0], lane);
-    const HugeDims hd = huge_dims(e);
-    double *wr        = vp.ws + e.woff;
+    auto hook = [&](int st) {
+      if (fw)
+        fetch_stage<true>(st, f, next, vp, nullptr, vp.nitems, &vp.counters[0], lane);
+    };
+    hook(0);
+    const VItem &it = slot.it;
+    const VDesc &e  = slot.e;
+    double *wr      = vp.ws + e.woff;
     if (it.kind == 0)
     {
       // phase 1: tail modes on head rows [lo, hi) -> the entry's region
-      GenView v1;
-      vp_view(v1, e, e.q, e.d - e.q);
-      v1.forward = e.fwd1;
-      vp_run(v1, it.hi - it.lo, x + (long long)it.lo * hd.Ntail,
-             wr + (long long)it.lo * hd.Mtail, ACC_STORE, smem, smem + e.mi, smem + 2 * e.mi, A,
-             tid, VP_THREADS, 0, hook);
+      vp_run<true>(slot.s.st, e.d - e.q, it.hi - it.lo, e.nin, e.nout,
+                   slot.ptr[6] + (long long)it.lo * e.nin, wr + (long long)it.lo * e.nout, smem,
+                   smem + e.mi, smem + 2 * e.mi, slot.ptr, tid, VP_THREADS, 0, hook);
       // vp_run ended with a block barrier: every store of the chunk is issued
       if (tid == 0)
       {
@@ -472,7 +480,7 @@ __global__ void __launch_bounds__(VP_THREADS, VP_MINB)
     else
     {
       // phase 2: head modes on column tile lo of the region -> y
-      if (!ready && !dead && !vp_wait_chunks(vp, it.e, e.nchunk, &s_flag, tid))
+      if (!slot.ready && !dead && !vp_wait_chunks(vp, it.e, e.nchunk, &s_flag, tid))
         dead = true;
       if (dead)
       {
@@ -484,12 +492,10 @@ __global__ void __launch_bounds__(VP_THREADS, VP_MINB)
         }
         continue;
       }
-      GenView v2;
-      vp_view(v2, e, 0, e.q);
-      v2.forward   = e.fwd2;
       const int c0 = it.lo * e.C;
-      vp_run_tile(v2, wr + c0, hd.Mtail, e.C, min((int)e.C, hd.Mtail - c0), y + c0, hd.Mtail,
-                  smem, smem + e.mi2, smem + 2 * e.mi2, A, tid, hook);
+      vp_run_tile(slot.s.st + (e.d - e.q), e.q, e.hin, e.hout, wr + c0, e.nout, e.C,
+                  min((int)e.C, e.nout - c0), const_cast<double *>(slot.ptr[7]) + c0, e.nout,
+                  smem, smem + e.mi2, smem + 2 * e.mi2, slot.ptr, tid, hook);
     }
   }
   __syncthreads();
@@ -512,6 +518,7 @@ struct kron_vplan_st
   int nhuge, nblock, nhalf, nquad, nwarp;
   int nitems;
   VDesc *d_desc;
+  VSteps *d_steps;
   VItem *d_items;
   int *d_counters;            // NCOUNT work counters + one chunk counter per huge entry
   double flops;
@@ -560,7 +567,7 @@ bool plan_huge(int d, const int *m, const int *n, long long budget, HugeSplit &b
       a1 += (long long)m[l] * n[l];
       Mtail *= m[l];
     }
-    const long long R = (budget - even(a1) - 2) / (2 * r1);
+    const long long R = (budget - even(a1) - 8) / (2 * r1);
     const long long C = std::min<long long>({255, Mtail, (budget - even(a2) - 2) / (2 * r2)});
     if (R < 1 || C < 1)
       continue;
@@ -587,10 +594,12 @@ extern "C" int kron_vplan_create(kron_vplan_t *plan, int batchCount, int const s
   *plan = nullptr;
   const DeviceInfo &di = device_info();
   // shared elements per block: two blocks per SM (1 KB of each block's share
-  // is reserved by the hardware; 2 KB cover the kernel's own variables)
+  // is reserved by the hardware; 4 KB cover the kernel's own variables)
   const long long budget =
-      (std::min<long long>(di.max_smem_optin, di.smem_per_sm / VP_MINB - 1024) - 2048) / 8 & ~1LL;
+      (std::min<long long>(di.max_smem_optin, di.smem_per_sm / VP_MINB - 1024) - 4096) / 8 & ~1LL;
+  static_assert(sizeof(NextSlot) * 2 * VP_WARPS + 64 <= 4096, "the kernel's own variables");
   std::vector<VDesc> cls[NCLS];
+  std::vector<VSteps> stp[NCLS];
   std::vector<double> cost[NCLS];
   double total_flops = 0.0;
   for (int k = 0; k < batchCount; k++)
@@ -609,13 +618,13 @@ extern "C" int kron_vplan_create(kron_vplan_t *plan, int batchCount, int const s
       n[l] = s[2 + 2 * l];
       if (m[l] < 1 || n[l] < 1 || m[l] > 255 || n[l] > 255)
         return KRON_ERROR_INVALID_VALUE;
-      e.m[l] = (unsigned char)m[l];
-      e.n[l] = (unsigned char)n[l];
     }
     e.d              = (unsigned char)d;
     const bool fwd   = choose_forward(d, m, n);
-    e.fwd            = fwd ? 1 : 0;
-    const long long mi = even(max_intermediate(d, m, n, fwd));
+    // two more: x starts at the offset it has in a 16-byte unit
+    const long long mi = even(max_intermediate(d, m, n, fwd)) + 2;
+    VSteps vs;
+    std::memset(&vs, 0, sizeof(vs));
     const double fl  = std::min(flops_forward(d, m, n), flops_backward(d, m, n));
     total_flops += fl;
     long long asz = 0;
@@ -623,7 +632,7 @@ extern "C" int kron_vplan_create(kron_vplan_t *plan, int batchCount, int const s
       asz += (long long)m[l] * n[l];
     const long long need = 2 * mi + even(asz);
     int c;
-    if (mi <= WARP_MAX && 2 * WARP_MAX + even(asz) <= (budget / VP_WARPS & ~1LL))
+    if (mi <= WARP_MAX && 2 * mi + even(asz) <= (budget / VP_WARPS & ~1LL))
       c = CLS_WARP;
     else if (need <= (budget / 4 & ~1LL))
       c = CLS_QUAD;
@@ -639,29 +648,44 @@ extern "C" int kron_vplan_create(kron_vplan_t *plan, int batchCount, int const s
         return KRON_ERROR_NOT_SUPPORTED;
       e.q    = (unsigned char)hs.q;
       e.C    = (unsigned char)hs.C;
-      e.fwd1 = (unsigned char)hs.fwd1;
-      e.fwd2 = (unsigned char)hs.fwd2;
-      long long Nhead = 1;
-      for (int l = 0; l < hs.q; l++)
-        Nhead *= n[l];
+      e.nin = e.nout = e.hin = e.hout = 1;
+      for (int l = 0; l < d; l++)
+      {
+        (l < hs.q ? e.hin : e.nin) *= n[l];
+        (l < hs.q ? e.hout : e.nout) *= m[l];
+      }
+      rect_plan(vs.st, d - hs.q, m + hs.q, n + hs.q, hs.q, hs.fwd1 != 0, 1);
+      rect_plan(vs.st + (d - hs.q), hs.q, m, n, 0, hs.fwd2 != 0, hs.C);
       // chunks of equal size, at most R rows each
-      const long long nchunk = (Nhead + hs.R - 1) / hs.R;
-      const long long R      = (Nhead + nchunk - 1) / nchunk;
-      e.R      = (unsigned short)R;
+      const long long nchunk = (e.hin + hs.R - 1) / hs.R;
+      const long long R      = (e.hin + nchunk - 1) / nchunk;
+      e.R      = (int)R;
       e.nchunk = (int)nchunk;
-      e.mi     = (int)even(R * hs.mi1);
+      e.mi     = (int)even(R * hs.mi1) + 2;
       e.mi2    = (int)even(hs.C * hs.mi2);
     }
     if (c != CLS_HUGE)
-      e.mi = (c == CLS_WARP) ? WARP_MAX : (int)mi;
+    {
+      e.mi  = (int)mi;
+      e.nin = e.nout = 1;
+      for (int l = 0; l < d; l++)
+      {
+        e.nin *= n[l];
+        e.nout *= m[l];
+      }
+      rect_plan(vs.st, d, m, n, 0, fwd, 1);
+    }
     cls[c].push_back(e);
+    stp[c].push_back(vs);
     cost[c].push_back(fl);
   }
   kron_vplan_st *pl = new (std::nothrow) kron_vplan_st();
   if (!pl)
     return KRON_ERROR_ALLOC;
   std::vector<VDesc> all;
+  std::vector<VSteps> steps;
   all.reserve(batchCount);
+  steps.reserve(batchCount);
   for (int c : {CLS_HUGE, CLS_BLOCK, CLS_HALF, CLS_QUAD, CLS_WARP})
   {
     std::vector<int> order(cls[c].size());
@@ -669,7 +693,10 @@ extern "C" int kron_vplan_create(kron_vplan_t *plan, int batchCount, int const s
     std::stable_sort(order.begin(), order.end(),
                      [&](int a, int b) { return cost[c][a] > cost[c][b]; });
     for (int i : order)
+    {
       all.push_back(cls[c][i]);
+      steps.push_back(stp[c][i]);
+    }
   }
   pl->batch  = batchCount;
   pl->nhuge  = (int)cls[CLS_HUGE].size();
@@ -697,11 +724,8 @@ extern "C" int kron_vplan_create(kron_vplan_t *plan, int batchCount, int const s
   long long live     = 0;
   long long woff     = 0;
   auto emit_tiles = [&](const Pending &p) {
-    const VDesc &e = all[p.e];
-    long long Mtail = 1;
-    for (int l = e.q; l < e.d; l++)
-      Mtail *= e.m[l];
-    const long long nt = (Mtail + e.C - 1) / e.C;
+    const VDesc &e     = all[p.e];
+    const long long nt = (e.nout + e.C - 1) / e.C;
     for (long long t = 0; t < nt; t++)
       items.push_back(VItem{p.e, (int)t, (int)t + 1, 1});
     live -= p.elems;
@@ -710,11 +734,7 @@ extern "C" int kron_vplan_create(kron_vplan_t *plan, int batchCount, int const s
   {
     VDesc &e = all[i];
     e.woff   = woff;
-    long long Nhead = 1, Mtail = 1;
-    for (int l = 0; l < e.q; l++)
-      Nhead *= e.n[l];
-    for (int l = e.q; l < e.d; l++)
-      Mtail *= e.m[l];
+    const long long Nhead = e.hin, Mtail = e.nout;
     const long long region = (Nhead * Mtail + 15) & ~15LL;
     woff += region;
     for (long long h0 = 0; h0 < Nhead; h0 += e.R)
@@ -737,14 +757,17 @@ extern "C" int kron_vplan_create(kron_vplan_t *plan, int batchCount, int const s
                      (pl->nquad + 3) / 4 + (pl->nwarp + VP_WARPS - 1) / VP_WARPS);
   pl->exec       = nullptr;
   pl->d_desc     = nullptr;
+  pl->d_steps    = nullptr;
   pl->d_items    = nullptr;
   pl->d_counters = nullptr;
   const size_t ncount = NCOUNT + (size_t)pl->nhuge;
   if (kron::dev_malloc((void **)&pl->d_counters, ncount * sizeof(int)) != cudaSuccess ||
       (batchCount > 0 && kron::dev_malloc((void **)&pl->d_desc, sizeof(VDesc) * batchCount) != cudaSuccess) ||
+      (batchCount > 0 && kron::dev_malloc((void **)&pl->d_steps, sizeof(VSteps) * batchCount) != cudaSuccess) ||
       (!items.empty() && kron::dev_malloc((void **)&pl->d_items, sizeof(VItem) * items.size()) != cudaSuccess))
   {
     kron::dev_free(pl->d_items);
+    kron::dev_free(pl->d_steps);
     kron::dev_free(pl->d_desc);
     kron::dev_free(pl->d_counters);
     delete pl;
@@ -752,10 +775,13 @@ extern "C" int kron_vplan_create(kron_vplan_t *plan, int batchCount, int const s
   }
   if ((batchCount > 0 && cudaMemcpy(pl->d_desc, all.data(), sizeof(VDesc) * batchCount,
                                     cudaMemcpyHostToDevice) != cudaSuccess) ||
+      (batchCount > 0 && cudaMemcpy(pl->d_steps, steps.data(), sizeof(VSteps) * batchCount,
+                                    cudaMemcpyHostToDevice) != cudaSuccess) ||
       (!items.empty() && cudaMemcpy(pl->d_items, items.data(), sizeof(VItem) * items.size(),
                                     cudaMemcpyHostToDevice) != cudaSuccess))
   {
     kron::dev_free(pl->d_items);
+    kron::dev_free(pl->d_steps);
     kron::dev_free(pl->d_desc);
     kron::dev_free(pl->d_counters);
     delete pl;
@@ -772,6 +798,7 @@ extern "C" int kron_vplan_destroy(kron_vplan_t plan)
   if (plan->exec)
     cudaGraphExecDestroy(plan->exec);
   kron::dev_free(plan->d_items);
+  kron::dev_free(plan->d_steps);
   kron::dev_free(plan->d_desc);
   kron::dev_free(plan->d_counters);
   delete plan;
@@ -792,6 +819,7 @@ static int vplan_launch_all(kron_vplan_t pl, double const *const *A, double **X,
   VParams vp;
   std::memset(&vp, 0, sizeof(vp));
   vp.desc     = pl->d_desc;
+  vp.steps    = pl->d_steps;
   vp.items    = pl->d_items;
   vp.nhuge    = pl->nhuge;
   vp.nblock   = pl->nblock;
