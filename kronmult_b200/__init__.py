@@ -129,12 +129,27 @@ def declared_symbols():
 
 
 # ---------------------------------------------------------------- torch helpers
-def _torch():
-    import torch
+_TORCH = None  # torch, once a CUDA device was seen
+_FN = {}       # the library's functions by name
 
-    if not torch.cuda.is_available():
-        raise RuntimeError("kronmult_b200 needs a CUDA device")
-    return torch
+
+def _torch():
+    global _TORCH
+    if _TORCH is None:
+        import torch
+
+        if not torch.cuda.is_available():
+            raise RuntimeError("kronmult_b200 needs a CUDA device")
+        torch.cuda.init()
+        _TORCH = torch
+    return _TORCH
+
+
+def _fn(name):
+    f = _FN.get(name)
+    if f is None:
+        f = _FN[name] = getattr(lib(), name)
+    return f
 
 
 def _ptr(t):
@@ -142,9 +157,17 @@ def _ptr(t):
 
 
 def _stream(stream):
-    torch = _torch()
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    # a call's host time is a few microseconds: the current stream's handle is
+    # taken straight from torch's C API (0.2 us; 3.1 us through a Stream
+    # object) where it has that function
+    torch = _TORCH or _torch()
+    if stream is not None:
+        return stream.cuda_stream
+    c = torch._C
+    try:
+        return c._cuda_getCurrentRawStream(c._cuda_getDevice())
+    except AttributeError:
+        return torch.cuda.current_stream().cuda_stream
 
 
 def _check(rc, what):
@@ -154,51 +177,66 @@ def _check(rc, what):
 
 def kronmult_batched(d, n, A, X, Y, W=None, stream=None):
     """Y(:,k) += kron(A_1..A_d)(k) X(:,k) -- kronmult{d}_batched."""
-    f = getattr(lib(), f"kronmult{d}_batched_async")
+    name = f"kronmult{d}_batched_async"
     batch = Y.numel() // (n ** d) if n else 0
-    _check(f(n, _ptr(A), _ptr(X), _ptr(Y), _ptr(W), batch, _stream(stream)),
-           f"kronmult{d}_batched")
+    rc = (_FN.get(name) or _fn(name))(n, _ptr(A), _ptr(X), Y.data_ptr(), _ptr(W), batch,
+                                      _stream(stream))
+    if rc:
+        _check(rc, f"kronmult{d}_batched")
 
 
 def kronmult_pbatched(d, n, A, pX, pY, pW=None, stream=None):
-    f = getattr(lib(), f"kronmult{d}_pbatched_async")
-    _check(f(n, _ptr(A), _ptr(pX), _ptr(pY), _ptr(pW), pX.numel(), _stream(stream)),
-           f"kronmult{d}_pbatched")
+    name = f"kronmult{d}_pbatched_async"
+    rc = (_FN.get(name) or _fn(name))(n, _ptr(A), _ptr(pX), _ptr(pY), _ptr(pW), pX.numel(),
+                                      _stream(stream))
+    if rc:
+        _check(rc, f"kronmult{d}_pbatched")
 
 
 def kronmult_xbatched(d, n, pA, lda, pX, pY, pW=None, subbatch=0, stream=None):
-    f = getattr(lib(), f"kronmult{d}_xbatched_async")
-    _check(f(n, _ptr(pA), lda, _ptr(pX), _ptr(pY), _ptr(pW), pX.numel(), subbatch,
-             _stream(stream)), f"kronmult{d}_xbatched")
+    name = f"kronmult{d}_xbatched_async"
+    rc = (_FN.get(name) or _fn(name))(n, _ptr(pA), lda, _ptr(pX), _ptr(pY), _ptr(pW), pX.numel(),
+                                      subbatch, _stream(stream))
+    if rc:
+        _check(rc, f"kronmult{d}_xbatched")
 
 
 def kronmult_vbatched(m, n, pA, pX, pY, W=None, stream=None):
     d = len(m)
-    f = getattr(lib(), f"kronmult{d}_vbatched_async")
+    name = f"kronmult{d}_vbatched_async"
     mn = []
     for a, b in zip(m, n):
         mn += [a, b]
     wbytes = 0 if W is None else W.numel() * W.element_size()
-    _check(f(*mn, _ptr(pA), _ptr(pX), _ptr(pY), _ptr(W), wbytes, pX.numel(), _stream(stream)),
-           f"kronmult{d}_vbatched")
+    rc = (_FN.get(name) or _fn(name))(*mn, _ptr(pA), _ptr(pX), _ptr(pY), _ptr(W), wbytes,
+                                      pX.numel(), _stream(stream))
+    if rc:
+        _check(rc, f"kronmult{d}_vbatched")
 
 
 def kgemm_batched(op, mm, nn, kk, alpha, pA, ldA, pB, ldB, beta, pC, ldC, stream=None):
-    f = getattr(lib(), f"kgemm_{op}_batched_async")
-    _check(f(mm, nn, kk, float(alpha), _ptr(pA), _ptr(ldA), _ptr(pB), _ptr(ldB), float(beta),
-             _ptr(pC), _ptr(ldC), pC.numel(), _stream(stream)), f"kgemm_{op}_batched")
+    name = f"kgemm_{op}_batched_async"
+    rc = (_FN.get(name) or _fn(name))(mm, nn, kk, float(alpha), _ptr(pA), _ptr(ldA), _ptr(pB),
+                                      _ptr(ldB), float(beta), _ptr(pC), _ptr(ldC), pC.numel(),
+                                      _stream(stream))
+    if rc:
+        _check(rc, f"kgemm_{op}_batched")
 
 
 def kronmult_batched_f32(d, n, A, X, Y, W=None, stream=None):
     batch = Y.numel() // (n ** d)
-    _check(lib().kronmult_batched_f32_async(d, n, _ptr(A), _ptr(X), _ptr(Y), _ptr(W), batch,
-                                            _stream(stream)), "kronmult_batched_f32")
+    rc = _fn("kronmult_batched_f32_async")(d, n, _ptr(A), _ptr(X), _ptr(Y), _ptr(W), batch,
+                                           _stream(stream))
+    if rc:
+        _check(rc, "kronmult_batched_f32")
 
 
 def kronmult_batched_split(d, n, A, X, Y, W=None, stream=None):
     batch = Y.numel() // (n ** d)
-    _check(lib().kronmult_batched_split_async(d, n, _ptr(A), _ptr(X), _ptr(Y), _ptr(W), batch,
-                                              _stream(stream)), "kronmult_batched_split")
+    rc = _fn("kronmult_batched_split_async")(d, n, _ptr(A), _ptr(X), _ptr(Y), _ptr(W), batch,
+                                             _stream(stream))
+    if rc:
+        _check(rc, "kronmult_batched_split")
 
 
 def measure_fp64_peak():
@@ -324,9 +362,9 @@ class Segments:
 
 
 def kronmult_xbatched_segmented(d, n, pA, lda, pX, pY, seg, pW=None, stream=None):
-    _check(lib().kronmult_xbatched_segmented_async(d, n, _ptr(pA), lda, _ptr(pX), _ptr(pY),
-                                                   _ptr(pW), pX.numel(), seg.handle,
-                                                   _stream(stream)),
+    _check(_fn("kronmult_xbatched_segmented_async")(d, n, _ptr(pA), lda, _ptr(pX), _ptr(pY),
+                                                    _ptr(pW), pX.numel(), seg.handle,
+                                                    _stream(stream)),
            "kronmult_xbatched_segmented")
 
 
@@ -359,7 +397,7 @@ class VPlan:
 
     def execute(self, pA, pX, pY, W=None, stream=None):
         wbytes = 0 if W is None else W.numel() * W.element_size()
-        _check(lib().kron_vplan_execute_async(self.handle, _ptr(pA), _ptr(pX), _ptr(pY), _ptr(W),
+        _check(_fn("kron_vplan_execute_async")(self.handle, _ptr(pA), _ptr(pX), _ptr(pY), _ptr(W),
                                               wbytes, _stream(stream)), "kron_vplan_execute")
 
     def close(self):

@@ -11,11 +11,14 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
+#include <cstring>
 #include <map>
 #include <mutex>
 #include <set>
 #include <utility>
 #include <vector>
+
+#include <unistd.h>
 
 #include "kron_launch.h"
 #include "kron_sq_table.cuh"
@@ -83,7 +86,12 @@ int cached_occupancy(const void *fn, int block, size_t smem, int *per_sm)
       return KRON_SUCCESS;
     }
   }
-  if (!attr.count({fn, dev}))
+  bool raised;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    raised = attr.count({fn, dev}) != 0;
+  }
+  if (!raised)
   {
     // dynamic + static shared memory may not exceed the opt-in maximum
     cudaFuncAttributes fa{};
@@ -641,6 +649,33 @@ int launch_variant(Params p, int prec, const Workspace &ws, int variant, int par
   }
 }
 
+// KRON_DISABLE_<variant> in the environment takes a variant out of the
+// built-in order.  One pass over the environment tells the usual call that
+// there is none (a getenv a variant cost more than the rest of the dispatch).
+static bool disable_variables()
+{
+  for (char **e = environ; e && *e; e++)
+    if ((*e)[0] == 'K' && std::strncmp(*e, "KRON_DISABLE_", 13) == 0)
+      return true;
+  return false;
+}
+
+static bool variant_disabled(int v)
+{
+  switch (v)
+  {
+  case VAR_MMA8: return std::getenv("KRON_DISABLE_MMA8") != nullptr;
+  case VAR_PIPE: return std::getenv("KRON_DISABLE_PIPE") != nullptr;
+  case VAR_RESIDENT: return std::getenv("KRON_DISABLE_RESIDENT") != nullptr;
+  case VAR_RING: return std::getenv("KRON_DISABLE_RING") != nullptr;
+  case VAR_SLAB: return std::getenv("KRON_DISABLE_SLAB") != nullptr;
+  case VAR_RECT: return std::getenv("KRON_DISABLE_RECT") != nullptr;
+  case VAR_BIG: return std::getenv("KRON_DISABLE_BIG") != nullptr;
+  case VAR_SPLIT_TC: return std::getenv("KRON_DISABLE_SPLIT_TC") != nullptr;
+  default: return false;
+  }
+}
+
 // FP32 d = 6, n = 6: a block an entry (resident) against a cluster of twelve
 // (slab), microseconds at 20 / 40 / 80 / 4096 entries: 19.8 / 20.5 / 20.9 /
 // 481 against 13.6 / 20.8 / 27.0 / 938.
@@ -680,18 +715,12 @@ int launch_kron(Params p, int prec, const Workspace &ws, cudaStream_t stream)
   // leaves the call to the next form)
   static const int order[] = {VAR_MMA8, VAR_PIPE, VAR_RESIDENT, VAR_RING, VAR_SLAB, VAR_SQ,
                               VAR_RECT, VAR_GEN,  VAR_BIG,  VAR_SPLIT_TC, VAR_LARGE};
+  const bool env = disable_variables();
   for (int v : order)
   {
     if ((v == VAR_RESIDENT && !prefer_resident(p)) || (v == VAR_RING && !prefer_ring(p)))
       continue;
-    if ((v == VAR_MMA8 && std::getenv("KRON_DISABLE_MMA8")) ||
-        (v == VAR_PIPE && std::getenv("KRON_DISABLE_PIPE")) ||
-        (v == VAR_RECT && std::getenv("KRON_DISABLE_RECT")) ||
-        (v == VAR_RESIDENT && std::getenv("KRON_DISABLE_RESIDENT")) ||
-        (v == VAR_RING && std::getenv("KRON_DISABLE_RING")) ||
-        (v == VAR_SLAB && std::getenv("KRON_DISABLE_SLAB")) ||
-        (v == VAR_BIG && std::getenv("KRON_DISABLE_BIG")) ||
-        (v == VAR_SPLIT_TC && std::getenv("KRON_DISABLE_SPLIT_TC")))
+    if (env && variant_disabled(v))
       continue;
     const int rc = launch_variant(p, prec, ws, v, 0, stream);
     if (rc != KRON_ERROR_NOT_SUPPORTED && !(v == VAR_RING && rc == KRON_ERROR_WORKSPACE))
