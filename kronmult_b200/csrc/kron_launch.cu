@@ -44,6 +44,8 @@ const DeviceInfo &device_info()
     info.sms = 148;
   if (info.max_smem_optin <= 0)
     info.max_smem_optin = (int)SMEM_OPTIN_MAX;
+  if (info.smem_per_sm <= 0)
+    info.smem_per_sm = 228 * 1024;
   cache.push_back(info);
   return cache.back();
 }

@@ -8,6 +8,8 @@
 // The factors lie in shared memory in the order of the steps.
 #pragma once
 
+#include <cmath>
+
 #include "kron_internal.cuh"
 
 namespace kron {
@@ -27,25 +29,25 @@ static_assert(sizeof(RectStep) == 16, "read as one 16-byte word");
 inline void rect_plan(RectStep *st, int dd, const int *m, const int *n, int mode0, bool forward,
                       int C)
 {
-  int dims[MAXD];
-  for (int q = 0; q < dd; q++)
-    dims[q] = n[q];
+  // `left`: the modes not yet applied (their input sizes), `done`: the applied
+  // ones (their output sizes), with the columns on the fastest side
+  unsigned left[MAXD + 1], done = forward ? 1u : (unsigned)C;
+  left[dd] = 1;
+  for (int s = dd - 1; s >= 0; s--)
+    left[s] = left[s + 1] * (unsigned)n[forward ? s : dd - 1 - s];
   for (int s = 0; s < dd; s++)
   {
-    const int q = forward ? s : dd - 1 - s;
-    long long outer = 1, inner = C;
-    for (int u = 0; u < q; u++)
-      outer *= dims[u];
-    for (int u = q + 1; u < dd; u++)
-      inner *= dims[u];
+    const int q          = forward ? s : dd - 1 - s;
+    const unsigned inner = forward ? left[s + 1] * (unsigned)C : done;
     st[s].inner = (int)inner;
-    st[s].nfib  = (int)(outer * inner);
-    st[s].magic = inner == 1 ? 0u : (unsigned)(((1ULL << 32) + inner - 1) / inner);
+    st[s].nfib  = (int)(forward ? done * inner : left[s + 1] * inner);
+    // exact in double: the quotient has 32 bits, its fraction at least 1 / inner
+    st[s].magic = inner == 1 ? 0u : (unsigned)std::ceil(4294967296.0 / inner);
     st[s].nq    = (unsigned char)n[q];
     st[s].mq    = (unsigned char)m[q];
     st[s].mode  = (unsigned char)(mode0 + q);
     st[s].pad   = 0;
-    dims[q]     = m[q];
+    done *= (unsigned)m[q];
   }
 }
 

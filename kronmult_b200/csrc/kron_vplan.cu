@@ -39,7 +39,6 @@
 #include <algorithm>
 #include <cstring>
 #include <new>
-#include <numeric>
 #include <vector>
 
 #include "kron_launch.h"
@@ -518,7 +517,7 @@ struct kron_vplan_st
   int nhuge, nblock, nhalf, nquad, nwarp;
   int nitems;
   VDesc *d_desc;
-  VSteps *d_steps;
+  VSteps *d_steps;            // in d_desc's block
   VItem *d_items;
   int *d_counters;            // NCOUNT work counters + one chunk counter per huge entry
   double flops;
@@ -534,6 +533,69 @@ struct kron_vplan_st
 namespace {
 
 long long even(long long v) { return (v + 1) & ~1LL; }
+
+// Alg. 993 order of an entry (forward only when strictly cheaper,
+// kronm.hpp:83-89), its flops and its largest intermediate, in one walk each
+// way.
+struct OrderCost
+{
+  bool forward;
+  double flops;
+  long long elems;
+};
+
+OrderCost order_cost(int d, const int *m, const int *n)
+{
+  // products of the sizes before and from each mode on
+  long long pm[MAXD + 1], pn[MAXD + 1], sm[MAXD + 1], sn[MAXD + 1];
+  pm[0] = pn[0] = sm[d] = sn[d] = 1;
+  for (int l = 0; l < d; l++)
+  {
+    pm[l + 1]     = pm[l] * m[l];
+    pn[l + 1]     = pn[l] * n[l];
+    sm[d - 1 - l] = sm[d - l] * m[d - 1 - l];
+    sn[d - 1 - l] = sn[d - l] * n[d - 1 - l];
+  }
+  long long fmax = pn[d], bmax = pn[d];
+  double ff = 0.0, fb = 0.0;
+  for (int l = 0; l < d; l++)
+  {
+    ff += 2.0 * (double)(pm[l + 1] * sn[l]);
+    fmax = std::max(fmax, pm[l + 1] * sn[l + 1]);
+    fb += 2.0 * (double)(pn[l + 1] * sm[l]);
+    bmax = std::max(bmax, pn[l] * sm[l]);
+  }
+  return ff < fb ? OrderCost{true, ff, fmax} : OrderCost{false, fb, bmax};
+}
+
+// Entries by falling cost, equal ones in entry order: a counting sort on the
+// bits of the (positive) cost as a float.
+struct Ranked
+{
+  float cost;
+  int k;
+};
+
+void sort_by_cost(std::vector<Ranked> &v)
+{
+  std::vector<Ranked> tmp(v.size());
+  for (int shift = 0; shift < 33; shift += 11)
+  {
+    unsigned count[2049] = {};
+    auto key = [&](const Ranked &r) {
+      unsigned b;
+      std::memcpy(&b, &r.cost, 4);
+      return (~b >> shift) & 2047u;
+    };
+    for (const Ranked &r : v)
+      count[key(r) + 1]++;
+    for (int i = 0; i < 2048; i++)
+      count[i + 1] += count[i];
+    for (const Ranked &r : v)
+      tmp[count[key(r)]++] = r;
+    v.swap(tmp);
+  }
+}
 
 // Two-phase split of a huge entry for a block of `budget` shared elements:
 // phase 1 applies modes [q, d) to chunks of R head rows, phase 2 modes
@@ -552,10 +614,9 @@ bool plan_huge(int d, const int *m, const int *n, long long budget, HugeSplit &b
   int best_c = 0;
   for (int q = 1; q < d; q++)
   {
-    const bool f1    = choose_forward(d - q, m + q, n + q);
-    const bool f2    = choose_forward(q, m, n);
-    const long long r1 = max_intermediate(d - q, m + q, n + q, f1);
-    const long long r2 = max_intermediate(q, m, n, f2);
+    const OrderCost o1 = order_cost(d - q, m + q, n + q);
+    const OrderCost o2 = order_cost(q, m, n);
+    const long long r1 = o1.elems, r2 = o2.elems;
     long long a1 = 0, a2 = 0, Nhead = 1, Mtail = 1;
     for (int l = 0; l < q; l++)
     {
@@ -575,8 +636,8 @@ bool plan_huge(int d, const int *m, const int *n, long long budget, HugeSplit &b
     const long long wsz = Nhead * Mtail;
     if (!found || cq > best_c || (cq == best_c && wsz < best_w))
     {
-      best = HugeSplit{q, (int)C, (int)std::min<long long>(R, 65535), f1 ? 1 : 0, f2 ? 1 : 0,
-                       r1, r2};
+      best = HugeSplit{q, (int)C, (int)std::min<long long>(R, 65535), o1.forward ? 1 : 0,
+                       o2.forward ? 1 : 0, r1, r2};
       best_c = cq;
       best_w = wsz;
       found  = true;
@@ -598,41 +659,40 @@ extern "C" int kron_vplan_create(kron_vplan_t *plan, int batchCount, int const s
   const long long budget =
       (std::min<long long>(di.max_smem_optin, di.smem_per_sm / VP_MINB - 1024) - 4096) / 8 & ~1LL;
   static_assert(sizeof(NextSlot) * 2 * VP_WARPS + 64 <= 4096, "the kernel's own variables");
-  std::vector<VDesc> cls[NCLS];
-  std::vector<VSteps> stp[NCLS];
-  std::vector<double> cost[NCLS];
+  // class and cost of every entry, then descriptors and steps in queue order
+  std::vector<Ranked> cls[NCLS];
+  std::vector<HugeSplit> splits; // of the huge entries, in entry order
+  std::vector<int> split_of(batchCount, -1);
   double total_flops = 0.0;
-  for (int k = 0; k < batchCount; k++)
-  {
+  int m[MAXD], n[MAXD];
+  auto shape_of = [&](int k) {
     const int *s = shapes + 13LL * k;
-    VDesc e;
-    std::memset(&e, 0, sizeof(e));
-    e.k     = k;
-    const int d = s[0];
-    if (d < 1 || d > MAXD)
-      return KRON_ERROR_INVALID_VALUE;
-    int m[MAXD], n[MAXD];
-    for (int l = 0; l < d; l++)
+    for (int l = 0; l < s[0]; l++)
     {
       m[l] = s[1 + 2 * l];
       n[l] = s[2 + 2 * l];
-      if (m[l] < 1 || n[l] < 1 || m[l] > 255 || n[l] > 255)
-        return KRON_ERROR_INVALID_VALUE;
     }
-    e.d              = (unsigned char)d;
-    const bool fwd   = choose_forward(d, m, n);
-    // two more: x starts at the offset it has in a 16-byte unit
-    const long long mi = even(max_intermediate(d, m, n, fwd)) + 2;
-    VSteps vs;
-    std::memset(&vs, 0, sizeof(vs));
-    const double fl  = std::min(flops_forward(d, m, n), flops_backward(d, m, n));
-    total_flops += fl;
+    return s[0];
+  };
+  for (int k = 0; k < batchCount; k++)
+  {
+    const int d = shapes[13LL * k];
+    if (d < 1 || d > MAXD)
+      return KRON_ERROR_INVALID_VALUE;
+    shape_of(k);
     long long asz = 0;
     for (int l = 0; l < d; l++)
+    {
+      if (m[l] < 1 || n[l] < 1 || m[l] > 255 || n[l] > 255)
+        return KRON_ERROR_INVALID_VALUE;
       asz += (long long)m[l] * n[l];
+    }
+    const OrderCost oc = order_cost(d, m, n);
+    total_flops += oc.flops;
+    const long long mi   = even(oc.elems) + 2;
     const long long need = 2 * mi + even(asz);
     int c;
-    if (mi <= WARP_MAX && 2 * mi + even(asz) <= (budget / VP_WARPS & ~1LL))
+    if (mi <= WARP_MAX && need <= (budget / VP_WARPS & ~1LL))
       c = CLS_WARP;
     else if (need <= (budget / 4 & ~1LL))
       c = CLS_QUAD;
@@ -646,16 +706,55 @@ extern "C" int kron_vplan_create(kron_vplan_t *plan, int batchCount, int const s
       HugeSplit hs;
       if (!plan_huge(d, m, n, budget, hs))
         return KRON_ERROR_NOT_SUPPORTED;
-      e.q    = (unsigned char)hs.q;
-      e.C    = (unsigned char)hs.C;
+      split_of[k] = (int)splits.size();
+      splits.push_back(hs);
+    }
+    cls[c].push_back(Ranked{(float)oc.flops, k});
+  }
+  kron_vplan_st *pl = new (std::nothrow) kron_vplan_st();
+  if (!pl)
+    return KRON_ERROR_ALLOC;
+  // descriptors, then steps: one device block
+  const size_t desc_bytes = (sizeof(VDesc) * batchCount + 15) / 16 * 16;
+  std::vector<unsigned char> host(desc_bytes + sizeof(VSteps) * batchCount);
+  VDesc *all    = reinterpret_cast<VDesc *>(host.data());
+  VSteps *steps = reinterpret_cast<VSteps *>(host.data() + desc_bytes);
+  int at        = 0;
+  for (int c : {CLS_HUGE, CLS_BLOCK, CLS_HALF, CLS_QUAD, CLS_WARP})
+  {
+    sort_by_cost(cls[c]);
+    for (const Ranked &r : cls[c])
+    {
+      VDesc &e     = all[at];
+      RectStep *st = steps[at].st;
+      at++;
+      const int d = shape_of(r.k);
+      e.k         = r.k;
+      e.d         = (unsigned char)d;
       e.nin = e.nout = e.hin = e.hout = 1;
+      if (c != CLS_HUGE)
+      {
+        for (int l = 0; l < d; l++)
+        {
+          e.nin *= n[l];
+          e.nout *= m[l];
+        }
+        const OrderCost oc = order_cost(d, m, n);
+        // two more: x starts at the offset it has in a 16-byte unit
+        e.mi = (int)even(oc.elems) + 2;
+        rect_plan(st, d, m, n, 0, oc.forward, 1);
+        continue;
+      }
+      const HugeSplit &hs = splits[split_of[r.k]];
+      e.q = (unsigned char)hs.q;
+      e.C = (unsigned char)hs.C;
       for (int l = 0; l < d; l++)
       {
         (l < hs.q ? e.hin : e.nin) *= n[l];
         (l < hs.q ? e.hout : e.nout) *= m[l];
       }
-      rect_plan(vs.st, d - hs.q, m + hs.q, n + hs.q, hs.q, hs.fwd1 != 0, 1);
-      rect_plan(vs.st + (d - hs.q), hs.q, m, n, 0, hs.fwd2 != 0, hs.C);
+      rect_plan(st, d - hs.q, m + hs.q, n + hs.q, hs.q, hs.fwd1 != 0, 1);
+      rect_plan(st + (d - hs.q), hs.q, m, n, 0, hs.fwd2 != 0, hs.C);
       // chunks of equal size, at most R rows each
       const long long nchunk = (e.hin + hs.R - 1) / hs.R;
       const long long R      = (e.hin + nchunk - 1) / nchunk;
@@ -663,39 +762,6 @@ extern "C" int kron_vplan_create(kron_vplan_t *plan, int batchCount, int const s
       e.nchunk = (int)nchunk;
       e.mi     = (int)even(R * hs.mi1) + 2;
       e.mi2    = (int)even(hs.C * hs.mi2);
-    }
-    if (c != CLS_HUGE)
-    {
-      e.mi  = (int)mi;
-      e.nin = e.nout = 1;
-      for (int l = 0; l < d; l++)
-      {
-        e.nin *= n[l];
-        e.nout *= m[l];
-      }
-      rect_plan(vs.st, d, m, n, 0, fwd, 1);
-    }
-    cls[c].push_back(e);
-    stp[c].push_back(vs);
-    cost[c].push_back(fl);
-  }
-  kron_vplan_st *pl = new (std::nothrow) kron_vplan_st();
-  if (!pl)
-    return KRON_ERROR_ALLOC;
-  std::vector<VDesc> all;
-  std::vector<VSteps> steps;
-  all.reserve(batchCount);
-  steps.reserve(batchCount);
-  for (int c : {CLS_HUGE, CLS_BLOCK, CLS_HALF, CLS_QUAD, CLS_WARP})
-  {
-    std::vector<int> order(cls[c].size());
-    std::iota(order.begin(), order.end(), 0);
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int a, int b) { return cost[c][a] > cost[c][b]; });
-    for (int i : order)
-    {
-      all.push_back(cls[c][i]);
-      steps.push_back(stp[c][i]);
     }
   }
   pl->batch  = batchCount;
@@ -757,31 +823,26 @@ extern "C" int kron_vplan_create(kron_vplan_t *plan, int batchCount, int const s
                      (pl->nquad + 3) / 4 + (pl->nwarp + VP_WARPS - 1) / VP_WARPS);
   pl->exec       = nullptr;
   pl->d_desc     = nullptr;
-  pl->d_steps    = nullptr;
   pl->d_items    = nullptr;
   pl->d_counters = nullptr;
   const size_t ncount = NCOUNT + (size_t)pl->nhuge;
   if (kron::dev_malloc((void **)&pl->d_counters, ncount * sizeof(int)) != cudaSuccess ||
-      (batchCount > 0 && kron::dev_malloc((void **)&pl->d_desc, sizeof(VDesc) * batchCount) != cudaSuccess) ||
-      (batchCount > 0 && kron::dev_malloc((void **)&pl->d_steps, sizeof(VSteps) * batchCount) != cudaSuccess) ||
+      (batchCount > 0 && kron::dev_malloc((void **)&pl->d_desc, host.size()) != cudaSuccess) ||
       (!items.empty() && kron::dev_malloc((void **)&pl->d_items, sizeof(VItem) * items.size()) != cudaSuccess))
   {
     kron::dev_free(pl->d_items);
-    kron::dev_free(pl->d_steps);
     kron::dev_free(pl->d_desc);
     kron::dev_free(pl->d_counters);
     delete pl;
     return KRON_ERROR_ALLOC;
   }
-  if ((batchCount > 0 && cudaMemcpy(pl->d_desc, all.data(), sizeof(VDesc) * batchCount,
-                                    cudaMemcpyHostToDevice) != cudaSuccess) ||
-      (batchCount > 0 && cudaMemcpy(pl->d_steps, steps.data(), sizeof(VSteps) * batchCount,
+  pl->d_steps = reinterpret_cast<VSteps *>(reinterpret_cast<unsigned char *>(pl->d_desc) + desc_bytes);
+  if ((batchCount > 0 && cudaMemcpy(pl->d_desc, host.data(), host.size(),
                                     cudaMemcpyHostToDevice) != cudaSuccess) ||
       (!items.empty() && cudaMemcpy(pl->d_items, items.data(), sizeof(VItem) * items.size(),
                                     cudaMemcpyHostToDevice) != cudaSuccess))
   {
     kron::dev_free(pl->d_items);
-    kron::dev_free(pl->d_steps);
     kron::dev_free(pl->d_desc);
     kron::dev_free(pl->d_counters);
     delete pl;
@@ -798,7 +859,6 @@ extern "C" int kron_vplan_destroy(kron_vplan_t plan)
   if (plan->exec)
     cudaGraphExecDestroy(plan->exec);
   kron::dev_free(plan->d_items);
-  kron::dev_free(plan->d_steps);
   kron::dev_free(plan->d_desc);
   kron::dev_free(plan->d_counters);
   delete plan;
