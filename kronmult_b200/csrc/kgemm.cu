@@ -6,8 +6,8 @@
 // atomics (C of different entries may alias, kgemm_nt.hpp:184-187),
 // beta == 0 stores without reading C, any other beta is a read-modify-write.
 //
-// Design: entries up to 64 x 64 x 64 run on the FP64 tensor cores, one entry
-// per block (kgemm_dmma_kernel, below).  Larger entries: one 64x64 output
+// Design: entries up to 64 x 64 x 64 run on the FP64 tensor cores
+// (kgemm_dmma_kernel, below).  Larger entries: one 64x64 output
 // tile per block (16x16 threads, 4x4 outputs per thread), K staged through
 // shared memory in steps of 16 with the operand transposes folded into the
 // staging loads, FP64 FMA accumulation.
@@ -133,17 +133,25 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---------------------------------------------------------------------------
-// Entries up to 64 x 64 x 64 on the FP64 tensor cores (mma.sync m8n8k4):
-// one entry per block of four warps at a time, warp w computing the 32 x 32
-// block of C at rows 32 (w / 2), columns 32 (w % 2) as 4 x 4 tiles of 8 x 8
-// held in fragments (D[g][2t], D[g][2t+1] per lane 4g + t), K in steps of 4
-// (A fragment op(A)[g][k], B fragment op(B)[k][g]).  op(A) and op(B) are
-// staged in shared memory, zero padded to whole tiles, in the orientation
-// that keeps both the global reads and the shared writes contiguous (stride
-// 68 doubles, so the fragment reads of either orientation are conflict free:
-// a half-warp's 16 lanes hit words 4g + t or 4t + g mod 16).
+// Entries up to 64 x 64 x 64 on the FP64 tensor cores (mma.sync m8n8k4).
+// WPE = 4: a block of four warps per entry, warp w computing the 32 x 32
+// block of C at rows 32 (w / 2), columns 32 (w % 2); WPE = 1 (mm, nn <= 32): a
+// warp per entry, so small entries fill an SM.  A warp holds 4 x 4 tiles of
+// 8 x 8 in fragments (D[g][2t], D[g][2t+1] per lane 4g + t), K in steps of 4
+// (A fragment op(A)[g][k], B fragment op(B)[k][g]).
+//
+// op(A) and op(B) are staged in shared memory line by line as they lie in
+// memory (lines of `len` contiguous elements), at a line stride of 4 mod 16
+// elements, so that the fragment reads of either orientation are conflict
+// free (a half-warp's 16 lanes hit words 4g + t or 4t + g mod 16).  The
+// padding to whole tiles is zeroed once: no copy ever writes there.  The next
+// entry's operands (copied 16 bytes at a time where alignment allows) take
+// off before the current entry's products when two stages leave enough blocks
+// an SM, else before its results go out; its pointers come an entry earlier
+// still.
+//
+// 64 x 64 x 64, 32768 entries, is bound by HBM (4.3 GB: 0.66 ms; FP64 0.46).
 constexpr int DM_THREADS = 128;
-constexpr int DM_S       = 68;
 constexpr int DM_MAX     = 64;
 
 __device__ __forceinline__ void dm_mma(double &d0, double &d1, double a, double b)
@@ -153,141 +161,242 @@ __device__ __forceinline__ void dm_mma(double &d0, double &d1, double a, double 
                : "d"(a), "d"(b));
 }
 
-// dst = *src (8 bytes) by an asynchronous copy, or 0 when !valid (zero
-// fill: nothing is read)
-__device__ __forceinline__ void dm_cp8(double *dst, const double *src, bool valid)
+// One operand: `lines` lines of `len` elements, staged at stride S; the magics
+// divide by len / 2 and by len (0 for a divisor of 1).
+struct DmOperand
 {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(s), "l"(src),
-               "r"(valid ? 8 : 0)
-               : "memory");
+  int lines, len, S;
+  unsigned magic2, magic1;
+};
+
+struct DmArgs
+{
+  int mm, nn, kk, batch;
+  DmOperand a, b;
+  int a_elems, stage_elems, stages; // shared elements: of op(A), of a stage
+  double alpha, beta;
+  double *const *A, *const *B, *const *C;
+  const int *ldA, *ldB, *ldC;
+};
+
+__device__ __forceinline__ void dm_copy(const DmOperand &o, double *dst, const double *src,
+                                        long long ld, int t, int G)
+{
+  if ((reinterpret_cast<uintptr_t>(src) & 15) == 0 && (ld & 1) == 0)
+  {
+    const int units = o.len >> 1;
+    for (int q = t; q < o.lines * units; q += G)
+    {
+      const int l = o.magic2 ? (int)__umulhi((unsigned)q, o.magic2) : q, u = q - l * units;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst + l * o.S + 2 * u)),
+                   "l"(src + l * ld + 2 * u)
+                   : "memory");
+    }
+    if (o.len & 1)
+      for (int l = t; l < o.lines; l += G)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst + l * o.S + o.len - 1)),
+                     "l"(src + l * ld + o.len - 1)
+                     : "memory");
+  }
+  else
+    for (int q = t; q < o.lines * o.len; q += G)
+    {
+      const int l = o.magic1 ? (int)__umulhi((unsigned)q, o.magic1) : q, u = q - l * o.len;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst + l * o.S + u)),
+                   "l"(src + l * ld + u)
+                   : "memory");
+    }
 }
 
-template <int OP> // 0 = nn, 1 = nt, 2 = tt
-__global__ void __launch_bounds__(DM_THREADS, 3)
-    kgemm_dmma_kernel(int mm, int nn, int kk, double alpha, double *const *Aarr,
-                      const int *ldAarr, double *const *Barr, const int *ldBarr, double beta,
-                      double *const *Carr, const int *ldCarr, int batch)
+struct DmEntry
 {
-  extern __shared__ double dm_smem[];
-  double *As = dm_smem;                // op(A): [k][i] (nn, nt) or [i][k] (tt)
-  double *Bs = dm_smem + DM_MAX * DM_S; // op(B): [j][k] (nn) or [k][j] (nt, tt)
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const double *A, *B;
+  double *C;
+  int ldA, ldB, ldC;
+};
+
+__device__ __forceinline__ void dm_entry(const DmArgs &p, int e, DmEntry &d)
+{
+  d.A   = p.A[e];
+  d.B   = p.B[e];
+  d.C   = p.C[e];
+  d.ldA = p.ldA[e];
+  d.ldB = p.ldB[e];
+  d.ldC = p.ldC[e];
+}
+
+template <int OP, int WPE> // OP: 0 = nn, 1 = nt, 2 = tt
+__global__ void __launch_bounds__(DM_THREADS, WPE == 4 ? 3 : 4)
+    kgemm_dmma_kernel(const __grid_constant__ DmArgs p)
+{
+  extern __shared__ __align__(16) double dm_smem[];
+  constexpr int G = 32 * WPE, NG = DM_THREADS / G;
+  const int grp = threadIdx.x / G, tid = threadIdx.x - grp * G;
+  const int warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int mt = (mm + 7) >> 3, nt = (nn + 7) >> 3, kt = (kk + 3) >> 2;
-  const int rows = mt * 8, cols = nt * 8, kp = kt * 4;
+  const int mt = (p.mm + 7) >> 3, nt = (p.nn + 7) >> 3, kt = (p.kk + 3) >> 2;
   const int m0 = 4 * (warp >> 1), n0 = 4 * (warp & 1); // first tile of this warp
-  constexpr bool A_KM = OP != 2; // A staged [k][i]
-  constexpr bool B_NK = OP == 0; // B staged [j][k]
+  constexpr bool A_KM = OP != 2; // A staged [k][i], else [i][k]
+  constexpr bool B_NK = OP == 0; // B staged [j][k], else [k][j]
+  double *base = dm_smem + (size_t)grp * p.stages * p.stage_elems;
+  auto sync    = [&]() {
+    if constexpr (WPE == 4)
+      __syncthreads();
+    else
+      __syncwarp();
+  };
 
-  for (int e = blockIdx.x; e < batch; e += gridDim.x)
+  for (int q = tid; q < p.stages * p.stage_elems; q += G)
+    base[q] = 0.0;
+  const int step = gridDim.x * NG;
+  int e          = blockIdx.x * NG + grp;
+  if (e >= p.batch)
+    return; // WPE = 1: the warps of a block share no barrier
+  sync();
+  DmEntry cur, nxt;
+  dm_entry(p, e, cur);
+  auto issue = [&](const DmEntry &d, int s) {
+    double *st = base + s * p.stage_elems;
+    dm_copy(p.a, st, d.A, d.ldA, tid, G);
+    dm_copy(p.b, st + p.a_elems, d.B, d.ldB, tid, G);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  issue(cur, 0);
+  if (e + step < p.batch)
+    dm_entry(p, e + step, nxt);
+  for (int s = 0;; s ^= p.stages - 1)
   {
-    const double *A     = Aarr[e];
-    const double *B     = Barr[e];
-    double *C           = Carr[e];
-    const long long lda = ldAarr[e], ldb = ldBarr[e], ldc = ldCarr[e];
-    __syncthreads(); // the previous entry's fragments are read
-    // every copy of the entry in flight at once (zero fill outside mm, nn, kk)
-    for (int q = tid; q < rows * kp; q += DM_THREADS)
+    const bool more = e + step < p.batch;
+    if (more && p.stages == 2)
     {
-      if constexpr (A_KM)
-      { // op(A)(i, k) = A[i + k lda]; consecutive threads walk i
-        const int i = q % rows, k = q / rows;
-        const bool ok = i < mm && k < kk;
-        dm_cp8(As + k * DM_S + i, ok ? A + i + k * lda : A, ok);
-      }
-      else
-      { // op(A)(i, k) = A[k + i lda]; consecutive threads walk k
-        const int k = q % kp, i = q / kp;
-        const bool ok = i < mm && k < kk;
-        dm_cp8(As + i * DM_S + k, ok ? A + k + i * lda : A, ok);
-      }
+      issue(nxt, s ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
     }
-    for (int q = tid; q < cols * kp; q += DM_THREADS)
-    {
-      if constexpr (B_NK)
-      { // op(B)(k, j) = B[k + j ldb]; consecutive threads walk k
-        const int k = q % kp, j = q / kp;
-        const bool ok = j < nn && k < kk;
-        dm_cp8(Bs + j * DM_S + k, ok ? B + k + j * ldb : B, ok);
-      }
-      else
-      { // op(B)(k, j) = B[j + k ldb]; consecutive threads walk j
-        const int j = q % cols, k = q / cols;
-        const bool ok = j < nn && k < kk;
-        dm_cp8(Bs + k * DM_S + j, ok ? B + j + k * ldb : B, ok);
-      }
-    }
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
+    else
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    sync();
 
+    const double *As = base + s * p.stage_elems, *Bs = As + p.a_elems;
+    const int sa = p.a.S, sb = p.b.S;
     double acc[4][4][2];
 #pragma unroll
     for (int a = 0; a < 4; a++)
 #pragma unroll
       for (int b = 0; b < 4; b++)
         acc[a][b][0] = acc[a][b][1] = 0.0;
-    for (int ks = 0; ks < kt; ks++)
+    if (m0 < mt && n0 < nt)
     {
-      const int k = ks * 4 + t;
-      double af[4], bf[4];
-#pragma unroll
-      for (int u = 0; u < 4; u++)
+      for (int ks = 0; ks < kt; ks++)
       {
-        const int r = (m0 + u) * 8 + g, c = (n0 + u) * 8 + g;
-        af[u] = (m0 + u < mt) ? (A_KM ? As[k * DM_S + r] : As[r * DM_S + k]) : 0.0;
-        bf[u] = (n0 + u < nt) ? (B_NK ? Bs[c * DM_S + k] : Bs[k * DM_S + c]) : 0.0;
+        const int k = ks * 4 + t;
+        double af[4], bf[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++)
+        {
+          const int r = (m0 + u) * 8 + g, c = (n0 + u) * 8 + g;
+          af[u] = (m0 + u < mt) ? (A_KM ? As[k * sa + r] : As[r * sa + k]) : 0.0;
+          bf[u] = (n0 + u < nt) ? (B_NK ? Bs[c * sb + k] : Bs[k * sb + c]) : 0.0;
+        }
+#pragma unroll
+        for (int a = 0; a < 4; a++)
+#pragma unroll
+          for (int b = 0; b < 4; b++)
+            if (m0 + a < mt && n0 + b < nt) // warp-uniform
+              dm_mma(acc[a][b][0], acc[a][b][1], af[a], bf[b]);
       }
-#pragma unroll
-      for (int a = 0; a < 4; a++)
-#pragma unroll
-        for (int b = 0; b < 4; b++)
-          if (m0 + a < mt && n0 + b < nt) // warp-uniform
-            dm_mma(acc[a][b][0], acc[a][b][1], af[a], bf[b]);
+    }
+    sync(); // the stage is read
+    double *C           = cur.C;
+    const long long ldc = cur.ldC;
+    if (more)
+    {
+      cur = nxt;
+      if (p.stages == 1)
+        issue(nxt, 0);
+      if (e + 2 * step < p.batch)
+        dm_entry(p, e + 2 * step, nxt);
     }
 #pragma unroll
     for (int a = 0; a < 4; a++)
+    {
+      const int i    = (m0 + a) * 8 + g;
+      const bool row = m0 + a < mt && i < p.mm;
+      double old[4][2];
+      if (p.beta != 1.0 && p.beta != 0.0)
+#pragma unroll
+        for (int b = 0; b < 4; b++)
+#pragma unroll
+          for (int pp = 0; pp < 2; pp++)
+          {
+            const int j = (n0 + b) * 8 + 2 * t + pp;
+            if (row && j < p.nn)
+              old[b][pp] = C[i + j * ldc];
+          }
 #pragma unroll
       for (int b = 0; b < 4; b++)
 #pragma unroll
         for (int pp = 0; pp < 2; pp++)
         {
-          const int i = (m0 + a) * 8 + g, j = (n0 + b) * 8 + 2 * t + pp;
-          if (m0 + a < mt && n0 + b < nt && i < mm && j < nn)
+          const int j = (n0 + b) * 8 + 2 * t + pp;
+          if (row && j < p.nn)
           {
             double *c      = C + i + j * ldc;
-            const double v = alpha * acc[a][b][pp];
-            if (beta == 1.0)
+            const double v = p.alpha * acc[a][b][pp];
+            if (p.beta == 1.0)
               atomicAdd(c, v);
-            else if (beta == 0.0)
+            else if (p.beta == 0.0)
               *c = v;
             else
-              *c = beta * (*c) + v;
+              *c = p.beta * old[b][pp] + v;
           }
         }
+    }
+    if (!more)
+      break;
+    e += step;
   }
 }
 
-template <int OP>
-int launch_dmma(int mm, int nn, int kk, double alpha, double *const *A, const int *ldA,
-                double *const *B, const int *ldB, double beta, double *const *C, const int *ldC,
-                int batch, cudaStream_t stream)
+DmOperand dm_operand(int lines, int len)
 {
-  const void *fn    = reinterpret_cast<const void *>(&kgemm_dmma_kernel<OP>);
-  const size_t smem = 2 * (size_t)DM_MAX * DM_S * sizeof(double);
-  int per_sm        = 1;
+  auto magic = [](int v) { return v <= 1 ? 0u : (unsigned)(((1ULL << 32) + v - 1) / v); };
+  // whole tiles of lines and of elements (8, or 4 along K), stride 4 mod 16
+  return DmOperand{lines, len, (len + 15) / 16 * 16 + 4, magic(len / 2), magic(len)};
+}
+
+template <int OP, int WPE>
+int launch_dmma(DmArgs p, cudaStream_t stream)
+{
+  const void *fn = reinterpret_cast<const void *>(&kgemm_dmma_kernel<OP, WPE>);
+  constexpr int NG = 4 / WPE;
+  // padded lines: tiles of 8 rows or columns, steps of 4 along K
+  auto lines = [](int n, bool along_k) { return along_k ? (n + 3) / 4 * 4 : (n + 7) / 8 * 8; };
+  p.a         = OP == 2 ? dm_operand(p.mm, p.kk) : dm_operand(p.kk, p.mm);
+  p.b         = OP == 0 ? dm_operand(p.nn, p.kk) : dm_operand(p.kk, p.nn);
+  p.a_elems   = lines(p.a.lines, OP != 2) * p.a.S;
+  p.stage_elems = p.a_elems + lines(p.b.lines, OP != 0) * p.b.S;
+  // two stages where they leave as many blocks an SM as the registers do
+  const size_t stage = (size_t)p.stage_elems * NG * 8;
+  const int blocks   = WPE == 4 ? 3 : 4;
+  p.stages           = blocks * (2 * stage + 1024) <= (size_t)device_info().smem_per_sm ? 2 : 1;
+  const size_t smem  = p.stages * stage;
+  int per_sm         = 1;
   if (cached_occupancy(fn, DM_THREADS, smem, &per_sm) != KRON_SUCCESS)
     return KRON_ERROR_LAUNCH;
-  const long long grid =
-      std::max<long long>(1, std::min<long long>(batch, (long long)device_info().sms * per_sm));
-  void *args[] = {&mm, &nn, &kk, &alpha, const_cast<double *const **>(&A),
-                  const_cast<const int **>(&ldA), const_cast<double *const **>(&B),
-                  const_cast<const int **>(&ldB), &beta, const_cast<double *const **>(&C),
-                  const_cast<const int **>(&ldC), &batch};
+  const long long grid = std::max<long long>(
+      1, std::min<long long>((p.batch + NG - 1) / NG, (long long)device_info().sms * per_sm));
+  void *args[] = {&p};
   return cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(DM_THREADS), args, smem, stream) ==
                  cudaSuccess
              ? KRON_SUCCESS
              : KRON_ERROR_LAUNCH;
+}
+
+template <int OP>
+int pick_dmma(const DmArgs &p, cudaStream_t stream)
+{
+  // a warp per entry where its 4 x 4 tiles cover C
+  return p.mm <= 32 && p.nn <= 32 ? launch_dmma<OP, 1>(p, stream) : launch_dmma<OP, 4>(p, stream);
 }
 
 } // namespace
@@ -302,11 +411,24 @@ int launch_kgemm(int op, int mm, int nn, int kk, double alpha, double *const *A,
   // tensor cores, one entry per block
   if (mm <= DM_MAX && nn <= DM_MAX && kk <= DM_MAX && !std::getenv("KRON_KGEMM_CUDA_CORES"))
   {
+    DmArgs p{};
+    p.mm    = mm;
+    p.nn    = nn;
+    p.kk    = kk;
+    p.batch = batch;
+    p.alpha = alpha;
+    p.beta  = beta;
+    p.A     = A;
+    p.B     = B;
+    p.C     = C;
+    p.ldA   = ldA;
+    p.ldB   = ldB;
+    p.ldC   = ldC;
     switch (op)
     {
-    case 0: return launch_dmma<0>(mm, nn, kk, alpha, A, ldA, B, ldB, beta, C, ldC, batch, stream);
-    case 1: return launch_dmma<1>(mm, nn, kk, alpha, A, ldA, B, ldB, beta, C, ldC, batch, stream);
-    case 2: return launch_dmma<2>(mm, nn, kk, alpha, A, ldA, B, ldB, beta, C, ldC, batch, stream);
+    case 0: return pick_dmma<0>(p, stream);
+    case 1: return pick_dmma<1>(p, stream);
+    case 2: return pick_dmma<2>(p, stream);
     default: return KRON_ERROR_INVALID_VALUE;
     }
   }
