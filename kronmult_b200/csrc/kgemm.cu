@@ -133,12 +133,11 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---------------------------------------------------------------------------
-// Entries up to 64 x 64 x 64 on the FP64 tensor cores (mma.sync m8n8k4).
-// WPE = 4: a block of four warps per entry, warp w computing the 32 x 32
-// block of C at rows 32 (w / 2), columns 32 (w % 2); WPE = 1 (mm, nn <= 32): a
-// warp per entry, so small entries fill an SM.  A warp holds 4 x 4 tiles of
-// 8 x 8 in fragments (D[g][2t], D[g][2t+1] per lane 4g + t), K in steps of 4
-// (A fragment op(A)[g][k], B fragment op(B)[k][g]).
+// Entries up to 64 x 64 x 64 on the FP64 tensor cores (mma.sync m16n8k8: half
+// the instructions of m8n8k4 at the same rate).  Four warps per entry, or one
+// (mm, nn <= 32), so that small entries fill an SM.  A warp holds TM x TN tiles
+// of 16 x 8 in fragments, 32 accumulators a lane: 32 x 32 of C, or 16 x 64, or 64 x
+// 16, whichever leaves the busiest warp least to do.
 //
 // op(A) and op(B) are staged in shared memory line by line as they lie in
 // memory (lines of `len` contiguous elements), at a line stride of 4 mod 16
@@ -150,15 +149,20 @@ __global__ void __launch_bounds__(256)
 // an SM, else before its results go out; its pointers come an entry earlier
 // still.
 //
-// 64 x 64 x 64, 32768 entries, is bound by HBM (4.3 GB: 0.66 ms; FP64 0.46).
+// Bound by HBM (64 x 64 x 64, 32768 entries: 4.3 GB, 0.66 ms; FP64 0.46).  Measured
+// there 1.20 -> 0.82 ms, 8 x 8 x 8 (60000 entries) 536 -> 52 us, 32 x 32 x 32 (60000)
+// 1017 -> 319 us, 58 x 35 x 29 (30000, beta = 0.5) 1382 -> 523 us, against one
+// entry a block whatever its size, loads, products and results in series, and two
+// divisions per copied element.
 constexpr int DM_THREADS = 128;
 constexpr int DM_MAX     = 64;
 
-__device__ __forceinline__ void dm_mma(double &d0, double &d1, double a, double b)
+__device__ __forceinline__ void dm_mma(double (&c)[4], const double (&a)[4], const double (&b)[2])
 {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
-               : "+d"(d0), "+d"(d1)
-               : "d"(a), "d"(b));
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, "
+               "{%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+               : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+               : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b[0]), "d"(b[1]));
 }
 
 // One operand: `lines` lines of `len` elements, staged at stride S; the magics
@@ -225,17 +229,22 @@ __device__ __forceinline__ void dm_entry(const DmArgs &p, int e, DmEntry &d)
   d.ldC = p.ldC[e];
 }
 
-template <int OP, int WPE> // OP: 0 = nn, 1 = nt, 2 = tt
-__global__ void __launch_bounds__(DM_THREADS, WPE == 4 ? 3 : 4)
+// OP: 0 = nn, 1 = nt, 2 = tt.  WM x WN warps an entry, each with TM x TN tiles;
+// FULL: every tile of every warp is whole.
+template <int OP, int WM, int WN, int TM, int TN, bool FULL>
+__global__ void __launch_bounds__(DM_THREADS, 3)
     kgemm_dmma_kernel(const __grid_constant__ DmArgs p)
 {
   extern __shared__ __align__(16) double dm_smem[];
-  constexpr int G = 32 * WPE, NG = DM_THREADS / G;
+  constexpr int WPE = WM * WN, G = 32 * WPE, NG = DM_THREADS / G;
   const int grp = threadIdx.x / G, tid = threadIdx.x - grp * G;
   const int warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int mt = (p.mm + 7) >> 3, nt = (p.nn + 7) >> 3, kt = (p.kk + 3) >> 2;
-  const int m0 = 4 * (warp >> 1), n0 = 4 * (warp & 1); // first tile of this warp
+  const int kt = (p.kk + 7) >> 3;
+  const int r0 = (warp / WN) * TM * 16, c0 = (warp % WN) * TN * 8; // this warp's part of C
+  // its tiles in use
+  const int na = FULL ? TM : min(TM, max(0, (p.mm - r0 + 15) >> 4));
+  const int nb = FULL ? TN : min(TN, max(0, (p.nn - c0 + 7) >> 3));
   constexpr bool A_KM = OP != 2; // A staged [k][i], else [i][k]
   constexpr bool B_NK = OP == 0; // B staged [j][k], else [k][j]
   double *base = dm_smem + (size_t)grp * p.stages * p.stage_elems;
@@ -276,37 +285,47 @@ __global__ void __launch_bounds__(DM_THREADS, WPE == 4 ? 3 : 4)
       asm volatile("cp.async.wait_group 0;" ::: "memory");
     sync();
 
-    const double *As = base + s * p.stage_elems, *Bs = As + p.a_elems;
-    const int sa = p.a.S, sb = p.b.S;
-    double acc[4][4][2];
+    // element (row r0 + g, k = t) of op(A), (k = t, column c0 + g) of op(B);
+    // steps between rows / columns and between ks
+    const int ar = A_KM ? 1 : p.a.S, ak = A_KM ? p.a.S : 1;
+    const int bc = B_NK ? p.b.S : 1, bk = B_NK ? 1 : p.b.S;
+    const double *Ap = base + s * p.stage_elems + (r0 + g) * ar + t * ak;
+    const double *Bp = base + s * p.stage_elems + p.a_elems + (c0 + g) * bc + t * bk;
+    double acc[TM][TN][4];
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int a = 0; a < TM; a++)
 #pragma unroll
-      for (int b = 0; b < 4; b++)
-        acc[a][b][0] = acc[a][b][1] = 0.0;
-    if (m0 < mt && n0 < nt)
+      for (int b = 0; b < TN; b++)
+        acc[a][b][0] = acc[a][b][1] = acc[a][b][2] = acc[a][b][3] = 0.0;
+    for (int ks = 0; ks < kt; ks++, Ap += 8 * ak, Bp += 8 * bk)
     {
-      for (int ks = 0; ks < kt; ks++)
-      {
-        const int k = ks * 4 + t;
-        double af[4], bf[4];
+      double af[TM][4], bf[TN][2];
 #pragma unroll
-        for (int u = 0; u < 4; u++)
+      for (int a = 0; a < TM; a++)
+        if (FULL || a < na)
         {
-          const int r = (m0 + u) * 8 + g, c = (n0 + u) * 8 + g;
-          af[u] = (m0 + u < mt) ? (A_KM ? As[k * sa + r] : As[r * sa + k]) : 0.0;
-          bf[u] = (n0 + u < nt) ? (B_NK ? Bs[c * sb + k] : Bs[k * sb + c]) : 0.0;
+          af[a][0] = Ap[a * 16 * ar];
+          af[a][1] = Ap[(a * 16 + 8) * ar];
+          af[a][2] = Ap[a * 16 * ar + 4 * ak];
+          af[a][3] = Ap[(a * 16 + 8) * ar + 4 * ak];
         }
 #pragma unroll
-        for (int a = 0; a < 4; a++)
+      for (int b = 0; b < TN; b++)
+        if (FULL || b < nb)
+        {
+          bf[b][0] = Bp[b * 8 * bc];
+          bf[b][1] = Bp[b * 8 * bc + 4 * bk];
+        }
 #pragma unroll
-          for (int b = 0; b < 4; b++)
-            if (m0 + a < mt && n0 + b < nt) // warp-uniform
-              dm_mma(acc[a][b][0], acc[a][b][1], af[a], bf[b]);
-      }
+      for (int b = 0; b < TN; b++)
+        if (FULL || b < nb) // warp-uniform
+#pragma unroll
+          for (int a = 0; a < TM; a++)
+            if (FULL || a < na)
+              dm_mma(acc[a][b], af[a], bf[b]);
     }
     sync(); // the stage is read
-    double *C           = cur.C;
+    double *C           = cur.C + (r0 + g) + (long long)(c0 + 2 * t) * cur.ldC;
     const long long ldc = cur.ldC;
     if (more)
     {
@@ -316,39 +335,54 @@ __global__ void __launch_bounds__(DM_THREADS, WPE == 4 ? 3 : 4)
       if (e + 2 * step < p.batch)
         dm_entry(p, e + 2 * step, nxt);
     }
+    // acc[a][b][2 h + pp]: row 16 a + 8 h + g, column 8 b + 2 t + pp
+    bool row[TM][2];
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int a = 0; a < TM; a++)
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+        row[a][h] = FULL || r0 + a * 16 + h * 8 + g < p.mm;
+    auto each = [&](int b, auto &&f) {
+      // the elements of column tile b that lie in C, down the columns
+#pragma unroll
+      for (int pp = 0; pp < 2; pp++)
+#pragma unroll
+        for (int a = 0; a < TM; a++)
+#pragma unroll
+          for (int h = 0; h < 2; h++)
+            if (FULL || (row[a][h] && c0 + b * 8 + 2 * t + pp < p.nn))
+              f(C + (b * 8 + pp) * ldc + a * 16 + h * 8, a, 2 * h + pp);
+    };
+    if (p.beta == 1.0)
     {
-      const int i    = (m0 + a) * 8 + g;
-      const bool row = m0 + a < mt && i < p.mm;
-      double old[4][2];
-      if (p.beta != 1.0 && p.beta != 0.0)
 #pragma unroll
-        for (int b = 0; b < 4; b++)
+      for (int b = 0; b < TN; b++)
+        if (FULL || b < nb)
+          each(b, [&](double *c, int a, int i) { atomicAdd(c, p.alpha * acc[a][b][i]); });
+    }
+    else if (p.beta == 0.0)
+    {
 #pragma unroll
-          for (int pp = 0; pp < 2; pp++)
-          {
-            const int j = (n0 + b) * 8 + 2 * t + pp;
-            if (row && j < p.nn)
-              old[b][pp] = C[i + j * ldc];
-          }
+      for (int b = 0; b < TN; b++)
+        if (FULL || b < nb)
+          each(b, [&](double *c, int a, int i) { *c = p.alpha * acc[a][b][i]; });
+    }
+    else
+    {
+      constexpr int BC = TM >= 4 ? 1 : 4 / TM; // four tiles of C are read at a time
 #pragma unroll
-      for (int b = 0; b < 4; b++)
-#pragma unroll
-        for (int pp = 0; pp < 2; pp++)
+      for (int b0 = 0; b0 < TN; b0 += BC)
+        if (FULL || b0 < nb)
         {
-          const int j = (n0 + b) * 8 + 2 * t + pp;
-          if (row && j < p.nn)
-          {
-            double *c      = C + i + j * ldc;
-            const double v = p.alpha * acc[a][b][pp];
-            if (p.beta == 1.0)
-              atomicAdd(c, v);
-            else if (p.beta == 0.0)
-              *c = v;
-            else
-              *c = p.beta * old[b][pp] + v;
-          }
+          double old[BC][TM][4];
+#pragma unroll
+          for (int b = 0; b < BC; b++)
+            each(b0 + b, [&](double *c, int a, int i) { old[b][a][i] = *c; });
+#pragma unroll
+          for (int b = 0; b < BC; b++)
+            each(b0 + b, [&](double *c, int a, int i) {
+              *c = p.beta * old[b][a][i] + p.alpha * acc[a][b0 + b][i];
+            });
         }
     }
     if (!more)
@@ -360,25 +394,24 @@ __global__ void __launch_bounds__(DM_THREADS, WPE == 4 ? 3 : 4)
 DmOperand dm_operand(int lines, int len)
 {
   auto magic = [](int v) { return v <= 1 ? 0u : (unsigned)(((1ULL << 32) + v - 1) / v); };
-  // whole tiles of lines and of elements (8, or 4 along K), stride 4 mod 16
   return DmOperand{lines, len, (len + 15) / 16 * 16 + 4, magic(len / 2), magic(len)};
 }
 
-template <int OP, int WPE>
+template <int OP, int WM, int WN, int TM, int TN, bool FULL>
 int launch_dmma(DmArgs p, cudaStream_t stream)
 {
-  const void *fn = reinterpret_cast<const void *>(&kgemm_dmma_kernel<OP, WPE>);
-  constexpr int NG = 4 / WPE;
-  // padded lines: tiles of 8 rows or columns, steps of 4 along K
-  auto lines = [](int n, bool along_k) { return along_k ? (n + 3) / 4 * 4 : (n + 7) / 8 * 8; };
+  const void *fn =
+      reinterpret_cast<const void *>(&kgemm_dmma_kernel<OP, WM, WN, TM, TN, FULL>);
+  constexpr int NG = 4 / (WM * WN);
+  // lines padded to whole tiles: 16 rows of A, 8 columns of B, 8 along K
+  auto up = [](int n, int q) { return (n + q - 1) / q * q; };
   p.a         = OP == 2 ? dm_operand(p.mm, p.kk) : dm_operand(p.kk, p.mm);
   p.b         = OP == 0 ? dm_operand(p.nn, p.kk) : dm_operand(p.kk, p.nn);
-  p.a_elems   = lines(p.a.lines, OP != 2) * p.a.S;
-  p.stage_elems = p.a_elems + lines(p.b.lines, OP != 0) * p.b.S;
+  p.a_elems   = up(p.a.lines, OP == 2 ? 16 : 8) * p.a.S;
+  p.stage_elems = p.a_elems + up(p.b.lines, 8) * p.b.S;
   // two stages where they leave as many blocks an SM as the registers do
   const size_t stage = (size_t)p.stage_elems * NG * 8;
-  const int blocks   = WPE == 4 ? 3 : 4;
-  p.stages           = blocks * (2 * stage + 1024) <= (size_t)device_info().smem_per_sm ? 2 : 1;
+  p.stages           = 3 * (2 * stage + 1024) <= (size_t)device_info().smem_per_sm ? 2 : 1;
   const size_t smem  = p.stages * stage;
   int per_sm         = 1;
   if (cached_occupancy(fn, DM_THREADS, smem, &per_sm) != KRON_SUCCESS)
@@ -395,8 +428,21 @@ int launch_dmma(DmArgs p, cudaStream_t stream)
 template <int OP>
 int pick_dmma(const DmArgs &p, cudaStream_t stream)
 {
-  // a warp per entry where its 4 x 4 tiles cover C
-  return p.mm <= 32 && p.nn <= 32 ? launch_dmma<OP, 1>(p, stream) : launch_dmma<OP, 4>(p, stream);
+  const int mt = (p.mm + 15) / 16, nt = (p.nn + 7) / 8;
+  if (p.mm == 32 && p.nn == 32)
+    return launch_dmma<OP, 1, 1, 2, 4, true>(p, stream);
+  if (mt <= 2 && nt <= 4)
+    return launch_dmma<OP, 1, 1, 2, 4, false>(p, stream);
+  if (p.mm == 64 && p.nn == 64)
+    return launch_dmma<OP, 2, 2, 2, 4, true>(p, stream);
+  // tiles of the busiest warp: two by two warps, four along the rows, four
+  // along the columns
+  const int t22 = std::min(mt, 2) * std::min(nt, 4), t41 = nt, t14 = mt * ((nt + 3) / 4);
+  if (t41 < t22 && t41 <= t14)
+    return launch_dmma<OP, 4, 1, 1, 8, false>(p, stream);
+  if (t14 < t22)
+    return launch_dmma<OP, 1, 4, 4, 2, false>(p, stream);
+  return launch_dmma<OP, 2, 2, 2, 4, false>(p, stream);
 }
 
 } // namespace
