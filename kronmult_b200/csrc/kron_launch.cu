@@ -685,11 +685,11 @@ static bool prefer_resident(const Params &p) { return p.eend - p.ebase >= 40; }
 
 // FP64 d = 6, n = 6: the ring's two phases are a serial chain of about 40 us,
 // a cluster of twelve an entry (slab) finishes 21 entries in 14 us;
-// microseconds at 80 / 160 / 320 / 4096 entries: 54 / 71 / 115 / 1204
+// microseconds at 80 / 160 / 320 / 4096 entries: 54 / 75 / 115 / 1190
 // against 39 / 70 / 132 / 1428.  n = 7, 8: the cluster two-phase kernel is
-// slower at every batch (3 entries, FP64: 136 against 44 us and 121 against
+// slower at every batch (3 entries, FP64: 136 against 35 us and 121 against
 // 60 us).
-static bool prefer_ring(const Params &p) { return p.n[0] > 6 || p.eend - p.ebase >= 160; }
+static bool prefer_ring(const Params &p) { return p.n[0] > 6 || p.eend - p.ebase >= 192; }
 
 int launch_kron(Params p, int prec, const Workspace &ws, cudaStream_t stream)
 {

@@ -12,7 +12,7 @@
 // parts: item g K + r is part r of entry g's phase 1 and part r of entry
 // (g - lag)'s phase 2.  Blocks take items in order from a device counter, so
 // an item waits only for items that running blocks already hold: phase 2 for
-// its entry's K phase-1 parts, lag groups back (normally long done), and
+// its entry's K phase-1 parts, lag entries back (normally long done), and
 // phase 1 for the ring slot of W it writes, last read by the entry `slots`
 // positions back.  W is a ring of `slots` vectors, a few tens of MB that stay
 // in the L2 cache however large the batch; no cluster barriers, and every SM
@@ -21,19 +21,16 @@
 //
 // The control words (queue, abort, and per slot the parts done of each phase,
 // counted up over the slot's generations) lie in the workspace vector after
-// the ring, zeroed by a small kernel ahead of this one.  A block publishes an
-// item's parts in the middle of the next item, when its stores have long
-// drained (a fence behind fresh stores and adds takes 2-3 us here), with one
-// fence for both counters and for the look at the next item's dependencies.  Waits are bounded (wait_limit() polls): a block that
+// the ring, zeroed by a small kernel ahead of this one.  Waits are bounded (wait_limit() polls): a block that
 // gives up records 1 in the device status word, raises the abort word, which
 // ends the others' waits, and leaves; y of the parts not done is untouched.
 //
 // Measured against what ran before (the cluster two-phase kernel, whose W
 // goes through HBM and back: 9.35 against 6.9 GB for 1024 entries of n = 8;
 // n = 6: the slab-cluster kernel with its side kernel):
-//   n = 6, 4096 entries  1.397 -> 1.289 ms (HBM alone 0.70)
-//   n = 7, 256 entries   0.465 -> 0.256 ms (HBM alone 0.11)
-//   n = 8, 1024 entries with aliasing outputs  2.049 -> 1.887 ms (FP64 tensor
+//   n = 6, 4096 entries  1.40 -> 1.23 ms (HBM alone 0.70)
+//   n = 7, 256 entries   0.465 -> 0.243 ms (HBM alone 0.11)
+//   n = 8, 1024 entries with aliasing outputs  2.05 -> 1.70 ms (FP64 tensor
 //   pipe alone 0.70, HBM 0.98)
 #include <algorithm>
 #include <cstdint>
@@ -172,13 +169,11 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src)
                "n"(BYTES)
                : "memory");
 }
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 // What a block knows of an item, in shared memory.
 struct Item
 {
   int idx;              // queue position (>= the total: no more work)
-  int ok;               // both dependencies were met when they were looked at
   int slot1, slot2;     // ring slots of phase 1 and phase 2, -1: no such part
   int need1, need2;     // counts that the slots' counters must have reached
   // 0-5: A_1..A_6 of the phase-1 entry, 6: its x, 7: its ring slot,
@@ -191,7 +186,6 @@ template <int K>
 __device__ __forceinline__ void item_plan(Item &it, int idx, int total, const RingArgs &w)
 {
   it.idx   = idx;
-  it.ok    = 0;
   it.slot1 = it.slot2 = -1;
   if (idx >= total)
     return;
@@ -210,166 +204,225 @@ __device__ __forceinline__ void item_plan(Item &it, int idx, int total, const Ri
   }
 }
 
-// The queue side of a block: item i in slot i % 3 of `items`, fetched two
-// items ahead by warp 0, a step at a time (the position when an item begins,
-// the pointers in its middle, the slot at its end).  Lane j < 16 of the warp
-// fetches pointer j, at base + index * stride, or what is stored there.
-template <typename T, int K>
-struct RingQueue
+// ---------------------------------------------------------------------------
+// Control warps, beside the group of warps that compute (a block, or a third of
+// one).  One takes items from the queue, starts their copies and waits for their
+// dependencies, an item ahead of the computing warps; another publishes parts,
+// so that its fences (2-3 us behind adds into y) hold nobody up.  Slot s
+// of two holds an item's operands; mbarriers:
+//   full[s]  the copies have landed (an arrival of each lane) and the
+//            dependencies are met (lane 0's).
+// Descriptions have four slots, so that the taker need not wait for the
+// publisher:
+//   done[d]  an arrival of each computing warp, behind its last access (of the
+//            taker in their place, for the end of the queue);
+//   read[d]  the publisher has read description d.
+// (No barrier can run two phases ahead of a thread that waits for it.)
+// All waits are bounded; when one runs out, the status and abort words are
+// raised and the computing warps find the end of the queue.
+constexpr int ITEM_SLOTS = 4;
+struct ControlBars
 {
-  Item *items;
-  int *s_dead;
-  int *ctl;
-  int total;
-  const char *base;  // warp 0
-  long long stride;
-  bool indirect;
-  int qn;            // lane 0: the queue position taken last
-  const void *pn;    // a pointer in flight
-  int pub1, pub2;    // thread 0: slots whose parts of the last item are unpublished
+  uint64_t full[2], done[ITEM_SLOTS], read[ITEM_SLOTS];
+};
 
-  __device__ __forceinline__ const void *pointer(int lane, int idx, const RingArgs &w)
+// one thread, before the block's first barrier; `warps` that compute
+__device__ __forceinline__ void control_init(ControlBars &bars, int warps)
+{
+  for (int s = 0; s < 2; s++)
+    mbar_init(&bars.full[s], 33);
+  for (int d = 0; d < ITEM_SLOTS; d++)
   {
-    int g = idx / K - (lane < 8 ? 0 : w.lag);
-    if (lane >= 16 || idx >= total || g < 0 || g >= w.nentries)
-      return nullptr;
-    if ((lane & 7) == 7)
-      g -= (int)__umulhi((unsigned)g, w.magic) * w.slots;
-    const char *a = base + g * stride;
-    return indirect ? *reinterpret_cast<const void *const *>(a) : a;
+    mbar_init(&bars.done[d], warps);
+    mbar_init(&bars.read[d], 1);
   }
-  __device__ __forceinline__ void start(const Params &p, const RingArgs &w, int tid)
+}
+
+// a bulk copy of this lane's that full[s] waits for
+__device__ __forceinline__ void bulk_into(uint64_t *bar, void *dst, const void *src, int bytes,
+                                          uint64_t pol)
+{
+  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)),
+               "r"(bytes)
+               : "memory");
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint "
+               "[%0], [%1], %2, [%3], %4;" ::"r"(smem_addr(dst)),
+               "l"(src), "r"(bytes), "r"(smem_addr(bar)), "l"(pol)
+               : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar)
+{
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
+}
+
+template <typename T, int K>
+struct RingControl
+{
+  // one warp, beside `warps` that compute; issue(item, slot, full) starts the
+  // copies of an item (whole warp)
+  template <typename Issue>
+  static __device__ __forceinline__ void run(const Params &p, const RingArgs &w, Item *items,
+                                             ControlBars &bars, int warps, int lane,
+                                             long long drain, const Issue &issue)
   {
-    ctl   = ring_ctl<T>(w);
-    total = (w.nentries + w.lag) * K;
-    pub1 = pub2 = -1;
-    if (tid < 32)
+    constexpr unsigned FULL = 0xffffffffu;
+    int *ctl        = ring_ctl<T>(w);
+    const int total = (w.nentries + w.lag) * K;
+    // lane j < 16 finds pointer j at base + index * stride, or stored there
+    const char *base = nullptr;
+    long long stride = 0;
+    bool indirect    = false;
+    const int m      = lane & 7;
+    if (m == 7)
     {
-      int q0 = 0, q1 = 0;
-      if (tid == 0)
-      {
-        q0 = atomicAdd(ctl + CTL_QUEUE, 2);
-        q1 = q0 + 1;
-        item_plan<K>(items[0], q0, total, w);
-        item_plan<K>(items[1], q1, total, w);
-      }
-      const int m = tid & 7;
-      if (m == 7)
-      {
-        indirect = w.ptrs != nullptr;
-        base     = reinterpret_cast<const char *>(indirect ? (const void *)w.ptrs : w.base);
-        stride   = indirect ? 8 : w.stride * (long long)sizeof(T);
-      }
-      else if (m == 6)
-      {
-        indirect = p.layout != LAYOUT_BATCHED;
-        if (indirect)
-          base = tid < 8 ? reinterpret_cast<const char *>(p.pX)
-                         : reinterpret_cast<const char *>(p.pY);
-        else
-          base = static_cast<const char *>(tid < 8 ? p.X : p.Y);
-        stride = indirect ? 8
-                          : (tid < 8 ? p.xstride : p.ystride) * (long long)sizeof(T);
-        base += p.ebase * stride;
-      }
+      indirect = w.ptrs != nullptr;
+      base     = reinterpret_cast<const char *>(indirect ? (const void *)w.ptrs : w.base);
+      stride   = indirect ? 8 : w.stride * (long long)sizeof(T);
+    }
+    else if (m == 6)
+    {
+      indirect = p.layout != LAYOUT_BATCHED;
+      if (indirect)
+        base = lane < 8 ? reinterpret_cast<const char *>(p.pX)
+                        : reinterpret_cast<const char *>(p.pY);
       else
-      {
-        indirect = p.layout != LAYOUT_BATCHED && p.layout != LAYOUT_PBATCHED;
-        const long long nn = (long long)p.n[0] * p.n[0] * (long long)sizeof(T);
-        stride   = indirect ? 8LL * p.apk : 6 * nn;
-        base     = indirect ? reinterpret_cast<const char *>(p.pA) + 8 * m
-                            : static_cast<const char *>(p.A) + m * nn;
-        base += p.ebase * stride;
-      }
-      q0 = __shfl_sync(0xffffffffu, q0, 0);
-      q1 = __shfl_sync(0xffffffffu, q1, 0);
-      const void *p0 = pointer(tid, q0, w), *p1 = pointer(tid, q1, w);
-      if (tid < 16)
-      {
-        items[0].ptr[tid] = const_cast<void *>(p0);
-        items[1].ptr[tid] = const_cast<void *>(p1);
-      }
+        base = static_cast<const char *>(lane < 8 ? p.X : p.Y);
+      stride = indirect ? 8 : (lane < 8 ? p.xstride : p.ystride) * (long long)sizeof(T);
+      base += p.ebase * stride;
     }
-    if (tid == 0)
-      *s_dead = 0;
-  }
-  // item i begins: take the position of item i + 2
-  __device__ __forceinline__ void take(int tid)
-  {
-    if (tid == 0)
-      qn = atomicAdd(ctl + CTL_QUEUE, 1);
-  }
-  // mid-item, warp 0: the pointers of item i + 2 take off
-  __device__ __forceinline__ void mid(const RingArgs &w, int tid)
-  {
-    if (tid < 32)
+    else
     {
-      qn = __shfl_sync(0xffffffffu, qn, 0);
-      pn = pointer(tid, qn, w);
+      indirect = p.layout != LAYOUT_BATCHED && p.layout != LAYOUT_PBATCHED;
+      const long long nn = (long long)p.n[0] * p.n[0] * (long long)sizeof(T);
+      stride   = indirect ? 8LL * p.apk : 6 * nn;
+      base     = indirect ? reinterpret_cast<const char *>(p.pA) + 8 * m
+                          : static_cast<const char *>(p.A) + m * nn;
+      base += p.ebase * stride;
     }
-  }
-  // thread 0, in the middle of an item, when the last item's accesses have
-  // drained: publish that item's parts and look at the next item's
-  // dependencies, under one fence
-  __device__ __forceinline__ void publish(Item *next)
-  {
-    bool ok = true;
-    if (next && next->idx < total)
+    int q = 0;
+    if (lane == 0)
+      q = atomicAdd(ctl + CTL_QUEUE, 1);
+    for (int j = 0;; j++)
     {
-      const int *a = ctl + ctl_phase2(max(next->slot1, 0));
-      const int *b = ctl + ctl_phase1(max(next->slot2, 0));
-      const int va = ld_relaxed(a), vb = ld_relaxed(b);
-      ok = (next->slot1 < 0 || va >= next->need1) && (next->slot2 < 0 || vb >= next->need2);
-    }
-    __threadfence();
-    if (pub1 >= 0)
-      red_relaxed(ctl + ctl_phase1(pub1));
-    if (pub2 >= 0)
-      red_relaxed(ctl + ctl_phase2(pub2));
-    pub1 = pub2 = -1;
-    if (next)
-      next->ok = ok ? 1 : 0;
-  }
-  // late in item i: item i + 2 takes its slot (warp 0)
-  __device__ __forceinline__ void late(Item &it, const RingArgs &w, int tid)
-  {
-    if (tid < 16)
-      it.ptr[tid] = const_cast<void *>(pn);
-    if (tid == 0)
-      item_plan<K>(it, qn, total, w);
-  }
-  // whole block, for an item whose dependencies were not met: false when the
-  // wait ran out (or another block's did)
-  __device__ __forceinline__ bool wait(const Item &it, const RingArgs &w, int tid)
-  {
-    if (tid == 0)
-    {
-      publish(nullptr);
-      const int *a = it.slot1 >= 0 ? ctl + ctl_phase2(it.slot1) : nullptr;
-      const int *b = it.slot2 >= 0 ? ctl + ctl_phase1(it.slot2) : nullptr;
-      long long polls = 0;
-      int dead        = 0;
-      while (true)
+      constexpr int D = ITEM_SLOTS;
+      Item &it      = items[j % D];
+      uint64_t *bar = &bars.full[j & 1];
+      const int idx = __shfl_sync(FULL, q, 0);
+      bool ok       = (j < 2 || mbar_wait_bounded(&bars.done[(j - 2) % D], ((j - 2) / D) & 1, drain)) &&
+                (j < D || mbar_wait_bounded(&bars.read[j % D], (j / D - 1) & 1, drain));
+      ok = __all_sync(FULL, ok);
+      if (lane == 0 && idx < total)
+        q = atomicAdd(ctl + CTL_QUEUE, 1);
+      if (lane == 0)
+        item_plan<K>(it, ok ? idx : total, total, w);
+      if (lane < 16)
       {
-        const int va = a ? ld_relaxed(a) : 0, vb = b ? ld_relaxed(b) : 0;
-        if ((!a || va >= it.need1) && (!b || vb >= it.need2))
-          break;
-        ++polls;
-        if (polls >= w.spin || (polls % 64 == 0 && ld_relaxed(ctl + CTL_ABORT) != 0))
+        int g         = idx / K - (lane < 8 ? 0 : w.lag);
+        const void *a = nullptr;
+        if (idx < total && g >= 0 && g < w.nentries)
         {
-          dead = 1;
+          if (m == 7)
+            g -= (int)__umulhi((unsigned)g, w.magic) * w.slots;
+          a = base + g * stride;
+          if (indirect)
+            a = *static_cast<const void *const *>(a);
+        }
+        it.ptr[lane] = const_cast<void *>(a);
+      }
+      // the slot's last readers come before the copies
+      fence_proxy_async();
+      __syncwarp();
+      const bool end = !ok || idx >= total;
+      if (!end)
+        issue(it, j & 1, bar);
+      asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar))
+                   : "memory");
+      bool met = true;
+      if (!end)
+      {
+        const int *a = it.slot1 >= 0 ? ctl + ctl_phase2(it.slot1) : nullptr;
+        const int *b = it.slot2 >= 0 ? ctl + ctl_phase1(it.slot2) : nullptr;
+        for (long long polls = 0;; polls++)
+        {
+          // every lane reads: one transaction, and no divergence
+          const int va = a ? ld_relaxed(a) : 0, vb = b ? ld_relaxed(b) : 0;
+          met          = __all_sync(FULL, (!a || va >= it.need1) && (!b || vb >= it.need2));
+          if (met || polls + 1 >= w.spin ||
+              (polls % 64 == 63 && __any_sync(FULL, ld_relaxed(ctl + CTL_ABORT) != 0)))
+            break;
+          __nanosleep(100);
+        }
+        __threadfence(); // what the others published is visible from here on
+      }
+      if (!ok || !met)
+      {
+        // the copies land in a buffer that nobody reads any more
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncwarp();
+        if (lane == 0)
+        {
           if (w.status)
             atomicExch(w.status, 1);
           atomicExch(ctl + CTL_ABORT, 1);
-          break;
+          it.idx = total;
         }
-        __nanosleep(200);
       }
-      __threadfence();
-      *s_dead = dead;
+      if (lane == 0)
+        mbar_arrive(bar);
+      if (end || !met)
+      {
+        if (lane == 0) // for the publisher
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&bars.done[j % D])),
+                       "r"(warps)
+                       : "memory");
+        return;
+      }
     }
-    __syncthreads();
-    return *s_dead == 0;
+  }
+
+  // One thread: publishes the parts of item j of a group once its computing
+  // warps are done with it.  0: not yet, 1: published, -1: the end of the queue.
+  static __device__ __forceinline__ int publish(const RingArgs &w, const Item *items,
+                                                ControlBars &bars, int j, int total)
+  {
+    if (!mbar_try_wait(&bars.done[j % ITEM_SLOTS], (j / ITEM_SLOTS) & 1))
+      return 0;
+    const Item &it = items[j % ITEM_SLOTS];
+    if (it.idx >= total)
+      return -1;
+    int *ctl     = ring_ctl<T>(w);
+    const int s1 = it.slot1, s2 = it.slot2;
+    mbar_arrive(&bars.read[j % ITEM_SLOTS]);
+    __threadfence();
+    if (s1 >= 0)
+      red_relaxed(ctl + ctl_phase1(s1));
+    if (s2 >= 0)
+      red_relaxed(ctl + ctl_phase2(s2));
+    return 1;
+  }
+  // the same for `groups` groups until all of them have come to the end
+  static __device__ __forceinline__ void publish_all(const RingArgs &w, const Item (*items)[ITEM_SLOTS],
+                                                     ControlBars *bars, int groups,
+                                                     long long drain)
+  {
+    const int total = (w.nentries + w.lag) * K;
+    int j[4] = {0, 0, 0, 0};
+    unsigned open = (1u << groups) - 1;
+    for (long long idle = 0; open && idle < drain; idle++)
+#pragma unroll
+      for (int g = 0; g < 4; g++)
+        if (g < groups && (open >> g & 1))
+        {
+          const int r = publish(w, items[g], bars[g], j[g], total);
+          if (r > 0)
+          {
+            j[g]++;
+            idle = 0;
+          }
+          else if (r < 0)
+            open &= ~(1u << g);
+        }
   }
 };
 
@@ -385,61 +438,103 @@ struct RingQueue
 // distinct banks (n = 6 FP64: 16 bytes after every fourth chunk; n = 8 FP32:
 // after every chunk; the others' chunk lengths are odd in 16-byte or element
 // units).
-template <typename T, int N, int R_, int THREADS_>
+//
+// A block is three such groups of four warps, which share nothing but the
+// control warps: three takers and a publisher.  One block an SM; the computing
+// warps take the registers that the control warps leave (160 of 128 + 128 / 3 a
+// thread: a fibre and a factor of n = 6 in FP64 are 144).
+template <typename T, int N, int R_>
 struct RingShape
 {
   static constexpr int N2 = N * N, LT = N2 * N2, LH = N2, L = LT * LH;
-  static constexpr int R = R_, THREADS = THREADS_;
+  static constexpr int R = R_, G = 128, GROUPS = 3, THREADS = 512;
   static constexpr int K   = (LH + R - 1) / R;
   static constexpr int CPI = (LT + K - 1) / K;
-  static constexpr int FIB = R * N2;
-  static_assert(FIB <= THREADS && CPI <= THREADS, "one fibre a thread");
+  static_assert(R * N2 <= G && CPI <= G, "one fibre a thread");
+  // setmaxnreg: the shares of a launch with 128 registers a thread
+  static constexpr int REGS = 160, CONTROL_REGS = 32;
+  static_assert(3 * G * REGS + G * CONTROL_REGS <= THREADS * 128, "register shares");
   static constexpr bool VEC   = N % 2 == 0; // chunks are whole 16-byte units
   static constexpr int V      = 16 / (int)sizeof(T);
   static constexpr int GROUP  = (N == 6 && sizeof(T) == 8) ? 4 : (N == 8 ? 1 : 0);
   static constexpr int ROW    = GROUP ? N2 * N2 + N2 / (GROUP ? GROUP : 1) * V : N2 * N2;
   static constexpr int BUF    = (R * ROW + 2 * V + 15) / 16 * 16; // + V: an unaligned start
   static constexpr int ASZ    = (6 * N2 + 3) / 4 * 4;             // A_1..A_6
-  static constexpr size_t OFF_A    = 0;
-  static constexpr size_t OFF_X    = 2 * (size_t)ASZ * sizeof(T);
-  static constexpr size_t SMEM     = OFF_X + 2 * (size_t)BUF * sizeof(T);
+  static constexpr int STAGE  = ASZ + BUF;                        // elements, two a group
+  static constexpr size_t SMEM = GROUPS * 2 * (size_t)STAGE * sizeof(T);
   __device__ static constexpr int chunk_off(int c)
   {
     return c * N2 + (GROUP ? c / (GROUP ? GROUP : 1) * V : 0);
   }
 };
 
-template <typename T, int N, int R, int THREADS, int MINB>
-__global__ void __launch_bounds__(THREADS, MINB)
-    kron_ring_kernel(const __grid_constant__ Params p, const __grid_constant__ RingArgs w)
+template <typename T, int N, int R>
+__global__ void __launch_bounds__(RingShape<T, N, R>::THREADS, 1)
+    kron_ring_kernel(const __grid_constant__ Params p, const __grid_constant__ RingArgs w,
+                     long long drain)
 {
-  using S          = RingShape<T, N, R, THREADS>;
+  using S          = RingShape<T, N, R>;
   constexpr int N2 = S::N2, LT = S::LT, LH = S::LH, K = S::K, V = S::V;
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ Item s_item[3];
-  __shared__ int s_dead;
-  const int tid = threadIdx.x;
-  auto stage_a  = [&](int b) { return reinterpret_cast<T *>(smem + S::OFF_A) + b * S::ASZ; };
-  auto stage_x  = [&](int b) { return reinterpret_cast<T *>(smem + S::OFF_X) + b * S::BUF; };
+  __shared__ Item s_item[S::GROUPS][ITEM_SLOTS];
+  __shared__ ControlBars s_bars[S::GROUPS];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // stage b of group gr: A_1..A_6, then the rows
+  auto stage_a = [&](int gr, int b) {
+    return reinterpret_cast<T *>(smem) + (gr * 2 + b) * S::STAGE;
+  };
   const RingPol pol = ring_policies();
-  const int ld      = p.layout == LAYOUT_XBATCHED ? p.lda : N;
+  const int total   = (w.nentries + w.lag) * K;
+  if (threadIdx.x == 0)
+  {
+    for (int gr = 0; gr < S::GROUPS; gr++)
+      control_init(s_bars[gr], 4);
+    fence_mbar_init();
+  }
+  __syncthreads();
 
-  // x rows and factors of item `it` into stage b.  A linear stage takes the
-  // rows at the offset that their start has in a 16-byte unit.
-  auto issue = [&](const Item &it, int b) {
-    if (it.slot1 >= 0)
+  if (warp >= 4 * S::GROUPS)
+  {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(S::CONTROL_REGS));
+    const int gr = warp - 4 * S::GROUPS;
+    if (gr == S::GROUPS)
     {
+      if (lane == 0)
+        RingControl<T, K>::publish_all(w, s_item, s_bars, S::GROUPS, drain);
+      return;
+    }
+    const int ld = p.layout == LAYOUT_XBATCHED ? p.lda : N;
+    // x rows and factors of an item; a linear stage takes the rows at the
+    // offset that their start has in a 16-byte unit
+    RingControl<T, K>::run(p, w, s_item[gr], s_bars[gr], 4, lane, drain, [&](const Item &it, int b,
+                                                                          uint64_t *bar) {
+      T *as = stage_a(gr, b);
+      // A_1, A_2 of the phase-2 entry, A_3..A_6 of the phase-1 entry
+      if (S::VEC && ld == N && lane < 6 && (lane < 2 ? it.slot2 : it.slot1) >= 0 &&
+          aligned16(it.ptr[lane < 2 ? 8 + lane : lane]))
+        bulk_into(bar, as + lane * N2, it.ptr[lane < 2 ? 8 + lane : lane], N2 * (int)sizeof(T),
+                  pol.keep);
+      else if (lane < 6 && (lane < 2 ? it.slot2 : it.slot1) >= 0)
+      {
+        const T *A = static_cast<const T *>(it.ptr[lane < 2 ? 8 + lane : lane]);
+        for (int j = 0; j < N; j++)
+          for (int i = 0; i < N; i++)
+            cp_async<sizeof(T)>(as + lane * N2 + j * N + i, A + i + (long long)j * ld);
+      }
+      if (it.slot1 < 0)
+        return;
       const int h0 = it.idx % K * R, ne = min(R, LH - h0) * LT;
       const T *src = static_cast<const T *>(it.ptr[6]) + (long long)h0 * LT;
-      T *buf       = stage_x(b);
+      T *buf       = as + S::ASZ;
       if constexpr (S::VEC)
       {
+        // a bulk copy per run of chunks between two paddings
+        constexpr int RUN = (S::GROUP ? S::GROUP : 1) * N2;
         if (aligned16(src))
-          for (int u = tid; u < ne / V; u += THREADS)
-            cp_async<16>(buf + u * V + (S::chunk_off(u * V / N2) - u * V / N2 * N2), src + u * V,
-                         pol.stream);
+          for (int c = lane; c < ne / RUN; c += 32)
+            bulk_into(bar, buf + c * (RUN + V), src + c * RUN, RUN * (int)sizeof(T), pol.stream);
         else
-          for (int u = tid; u < ne; u += THREADS)
+          for (int u = lane; u < ne; u += 32)
             cp_async<sizeof(T)>(buf + u + (S::chunk_off(u / N2) - u / N2 * N2), src + u);
       }
       else
@@ -447,60 +542,44 @@ __global__ void __launch_bounds__(THREADS, MINB)
         const int sh = (int)((reinterpret_cast<uintptr_t>(src) & 15) / sizeof(T));
         // units [u0, u1) lie whole in the rows; the ends go by elements
         const int u0 = (sh + V - 1) / V, u1 = (sh + ne) / V;
-        for (int u = u0 + tid; u < u1; u += THREADS)
-          cp_async<16>(buf + u * V, src - sh + u * V, pol.stream);
-        if (tid < u0 * V - sh)
-          cp_async<sizeof(T)>(buf + sh + tid, src + tid);
-        else if (tid >= 32 && u1 * V + tid - 32 < sh + ne)
-          cp_async<sizeof(T)>(buf + u1 * V + tid - 32, src + (u1 * V + tid - 32 - sh));
+        if (lane == 0)
+          bulk_into(bar, buf + u0 * V, src - sh + u0 * V, (u1 - u0) * 16, pol.stream);
+        if (lane < u0 * V - sh)
+          cp_async<sizeof(T)>(buf + sh + lane, src + lane);
+        if (u1 * V + lane < sh + ne)
+          cp_async<sizeof(T)>(buf + u1 * V + lane, src + (u1 * V + lane - sh));
       }
-    }
-    T *as = stage_a(b);
-    for (int q = tid; q < 6 * N2; q += THREADS)
-    {
-      // A_1, A_2 of the phase-2 entry, A_3..A_6 of the phase-1 entry
-      const int l = q / N2, ij = q - l * N2, j = ij / N, i = ij - j * N;
-      if (l < 2 ? it.slot2 >= 0 : it.slot1 >= 0)
-        cp_async<sizeof(T)>(as + q, static_cast<const T *>(it.ptr[l < 2 ? 8 + l : l]) + i +
-                                        (long long)j * ld);
-    }
-  };
+    });
+    return;
+  }
 
-  RingQueue<T, K> q;
-  q.items  = s_item;
-  q.s_dead = &s_dead;
-  q.start(p, w, tid);
-  __syncthreads();
-  if (s_item[0].idx < q.total)
-    issue(s_item[0], 0);
-  cp_async_wait();
-  __syncthreads();
-
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(S::REGS));
+  const int gr = warp >> 2, tid = threadIdx.x & 127;
+  const Item *items = s_item[gr];
+  ControlBars &bars = s_bars[gr];
   for (int i = 0;; ++i)
   {
-    const int b     = i & 1;
-    const Item &it  = s_item[i % 3];
-    if (it.idx >= q.total)
-      break;
-    if (!it.ok && !q.wait(it, w, tid))
-      break;
-    Item &next     = s_item[(i + 1) % 3];
+    const int b = i & 1;
+    if (!mbar_wait_bounded(&bars.full[b], (i >> 1) & 1, drain))
+    {
+      if (lane == 0 && w.status)
+        atomicExch(w.status, 1);
+      return;
+    }
+    const Item &it = items[i % ITEM_SLOTS];
+    if (it.idx >= total)
+      return;
     const int part = it.idx % K;
-    q.take(tid);
-    if (next.idx < q.total)
-      issue(next, b ^ 1);
-    const T *as = stage_a(b);
-
+    const T *as    = stage_a(gr, b);
     // ---- phase 1, modes 5 and 6 in place
-    const bool p1  = it.slot1 >= 0;
     const int h0   = part * R;
-    const int nfib = min(R, LH - h0) * N2;
-    T *xs          = stage_x(b);
+    const int nfib = it.slot1 >= 0 ? min(R, LH - h0) * N2 : 0;
+    T *xs          = stage_a(gr, b) + S::ASZ;
     if constexpr (!S::VEC)
-      if (p1)
+      if (nfib > 0)
         xs += (reinterpret_cast<uintptr_t>(static_cast<const T *>(it.ptr[6]) +
                                            (long long)h0 * LT) & 15) / sizeof(T);
-    if (p1 && tid < nfib)
+    if (tid < nfib)
     {
       T *c = xs + S::chunk_off(tid);
       T v[N2];
@@ -509,12 +588,9 @@ __global__ void __launch_bounds__(THREADS, MINB)
       apply_slow<T, N>(v, as + 4 * N2);
       store_chunk<T, N>(c, v);
     }
-    __syncthreads();
-    q.mid(w, tid);
-    if (tid == 0)
-      q.publish(&next);
+    asm volatile("bar.sync %0, 128;" ::"r"(gr + 1) : "memory");
     // ---- phase 1, modes 3 and 4; results into W
-    if (p1 && tid < nfib)
+    if (tid < nfib)
     {
       const int row = tid / N2, r = tid - row * N2;
       const T *c    = xs + row * S::ROW + r;
@@ -545,25 +621,21 @@ __global__ void __launch_bounds__(THREADS, MINB)
       for (int e = 0; e < N2; e++)
         y_add(y + (long long)e * LT, v[e], pol.stream);
     }
-    q.pub1 = it.slot1;
-    q.pub2 = it.slot2;
-    q.late(s_item[(i + 2) % 3], w, tid);
-    cp_async_wait();
-    __syncthreads();
+    __syncwarp();
+    if (lane == 0)
+      mbar_arrive(&bars.done[i % ITEM_SLOTS]);
   }
-  if (tid == 0)
-    q.publish(nullptr);
 }
 
 // ---------------------------------------------------------------------------
 // Tensor-core form (FP64, n = 7 and 8; n = 7 zero padded to 8): head = modes
-// 1..3, tail = modes 4..6, everything in mma.sync f64 fragments.
-//   phase 1: a warp takes a head row of n^3 elements (brought into its row
-//   buffer by cp.async during the item before), applies the three tail modes
-//   (kron8x3_tile) and stores the result into W;
-//   phase 2: a block takes 8 columns of W.  Warp j_1 loads its (j_2, j_3) x 8
-//   columns (64-byte row segments) with the columns on the fragments' G index
-//   and applies modes 3 and 2; the results change hands through shared memory
+// 1..3, tail = modes 4..6, everything in mma.sync f64 fragments.  Eight
+// computing warps and two control warps.
+//   phase 1: a warp takes a head row of n^3 elements, applies the three tail
+//   modes (kron8x3_tile) and stores the result into W;
+//   phase 2: a block takes 8 columns of W, which lie together (head row after
+//   head row).  Warp j_1 loads its (j_2, j_3) x 8 columns, 256 bytes at a time,
+//   with the columns on the fragments' G index and applies modes 3 and 2; the results change hands through shared memory
 //   (E[j_1][i_2][i_3][c]); warp i_2 applies mode 1 and adds into y.
 // E's strides spread the eight columns of four quads over distinct banks for
 // both its writes (i_2 = 2t+p) and its reads (j_1 = 2t+p).  A warp's slice of
@@ -573,14 +645,14 @@ struct RingMma
 {
   static constexpr int N3 = N * N * N, L = N3 * N3;
   static constexpr int K  = (N3 + 7) / 8;
-  static constexpr int THREADS = 256, MINB = 2;
+  static constexpr int WARPS = 8, THREADS = 32 * (WARPS + 2), MINB = 2; // two blocks an SM
   static constexpr int S2 = 66, S1 = 8 * S2 + 2; // strides of E's i_2 and j_1
   static constexpr int ASZ = 6 * N * N;
   static constexpr size_t OFF_E = (2 * (size_t)ASZ * 8 + 15) / 16 * 16;
-  // a warp's head row, at the offset that its start has in a 16-byte unit
-  static constexpr int ROW      = (N3 + 2 + 1) / 2 * 2;
+  // eight head rows, at the offset that their start has in a 16-byte unit
+  static constexpr int XLEN     = (8 * N3 + 2) / 2 * 2;
   static constexpr size_t OFF_X = OFF_E + 8 * (size_t)S1 * 8;
-  static constexpr size_t SMEM  = OFF_X + 8 * (size_t)ROW * 8;
+  static constexpr size_t SMEM  = OFF_X + 2 * (size_t)XLEN * 8;
 };
 
 template <int N>
@@ -593,73 +665,79 @@ __device__ __forceinline__ void frag_of(double (&b)[2], const double *A, int g, 
 
 template <int N>
 __global__ void __launch_bounds__(RingMma<N>::THREADS, RingMma<N>::MINB)
-    kron_ring_mma_kernel(const __grid_constant__ Params p, const __grid_constant__ RingArgs w)
+    kron_ring_mma_kernel(const __grid_constant__ Params p, const __grid_constant__ RingArgs w,
+                         long long drain)
 {
   using S          = RingMma<N>;
   constexpr int N2 = N * N, N3 = S::N3, K = S::K;
   extern __shared__ __align__(128) unsigned char smem[];
-  __shared__ Item s_item[3];
-  __shared__ int s_dead;
+  __shared__ Item s_item[ITEM_SLOTS];
+  __shared__ ControlBars s_bars;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, t = lane & 3;
-  double *E       = reinterpret_cast<double *>(smem + S::OFF_E);
-  double *scratch = E + warp * S::S1;
-  auto stage_a    = [&](int b) { return reinterpret_cast<double *>(smem) + b * S::ASZ; };
+  double *E     = reinterpret_cast<double *>(smem + S::OFF_E);
+  auto stage_a  = [&](int b) { return reinterpret_cast<double *>(smem) + b * S::ASZ; };
+  auto stage_x  = [&](int b) { return reinterpret_cast<double *>(smem + S::OFF_X) + b * S::XLEN; };
   const RingPol pol = ring_policies();
-  const int ld      = p.layout == LAYOUT_XBATCHED ? p.lda : N;
-
-  auto issue_a = [&](const Item &it, int b) {
-    double *as = stage_a(b);
-    for (int q = tid; q < 6 * N2; q += S::THREADS)
-    {
-      // A_1..A_3 of the phase-2 entry, A_4..A_6 of the phase-1 entry
-      const int l = q / N2, ij = q - l * N2, j = ij / N, i = ij - j * N;
-      if (l < 3 ? it.slot2 >= 0 : it.slot1 >= 0)
-        cp_async<8>(as + q, static_cast<const double *>(it.ptr[l < 3 ? 8 + l : l]) + i +
-                                (long long)j * ld);
-    }
-  };
-  // this warp's head row of `it` into its row buffer
-  double *row    = reinterpret_cast<double *>(smem + S::OFF_X) + warp * S::ROW;
-  auto issue_row = [&](const Item &it) {
-    const int h = it.idx % K * 8 + warp;
-    if (it.slot1 < 0 || h >= N3)
-      return;
-    const double *x = static_cast<const double *>(it.ptr[6]) + (long long)h * N3;
-    const int sh    = aligned16(x) ? 0 : 1;
-    const int u1    = (sh + N3) / 2; // units [sh, u1) lie whole in the row
-    for (int u = sh + lane; u < u1; u += 32)
-      cp_async<16>(row + 2 * u, x - sh + 2 * u, pol.stream);
-    if (sh && lane == 0)
-      cp_async<8>(row + 1, x);
-    if (((sh + N3) & 1) && lane == 1)
-      cp_async<8>(row + 2 * u1, x + N3 - 1);
-  };
-
-  RingQueue<double, K> q;
-  q.items  = s_item;
-  q.s_dead = &s_dead;
-  q.start(p, w, tid);
-  __syncthreads();
-  if (s_item[0].idx < q.total)
+  const int total   = (w.nentries + w.lag) * K;
+  if (tid == 0)
   {
-    issue_a(s_item[0], 0);
-    issue_row(s_item[0]);
+    control_init(s_bars, S::WARPS);
+    fence_mbar_init();
   }
-  cp_async_wait();
   __syncthreads();
 
+  if (warp == S::WARPS)
+  {
+    const int ld = p.layout == LAYOUT_XBATCHED ? p.lda : N;
+    RingControl<double, K>::run(
+        p, w, s_item, s_bars, S::WARPS, lane, drain, [&](const Item &it, int b, uint64_t *bar) {
+          double *as = stage_a(b);
+          for (int q = lane; q < 6 * N2; q += 32)
+          {
+            // A_1..A_3 of the phase-2 entry, A_4..A_6 of the phase-1 entry
+            const int l = q / N2, ij = q - l * N2, j = ij / N, i = ij - j * N;
+            if (l < 3 ? it.slot2 >= 0 : it.slot1 >= 0)
+              cp_async<8>(as + q, static_cast<const double *>(it.ptr[l < 3 ? 8 + l : l]) + i +
+                                      (long long)j * ld);
+          }
+          if (it.slot1 < 0)
+            return;
+          const int h0 = it.idx % K * 8, ne = min(8, N3 - h0) * N3;
+          const double *x = static_cast<const double *>(it.ptr[6]) + (long long)h0 * N3;
+          double *buf     = stage_x(b);
+          const int sh    = aligned16(x) ? 0 : 1;
+          const int u1    = (sh + ne) / 2; // units [sh, u1) lie whole in the rows
+          if (lane == 0)
+            bulk_into(bar, buf + 2 * sh, x - sh + 2 * sh, (u1 - sh) * 16, pol.stream);
+          if (sh && lane == 0)
+            cp_async<8>(buf + 1, x);
+          if (((sh + ne) & 1) && lane == 1)
+            cp_async<8>(buf + sh + ne - 1, x + ne - 1);
+        });
+    return;
+  }
+  if (warp > S::WARPS)
+  {
+    if (lane == 0)
+      RingControl<double, K>::publish_all(w, &s_item, &s_bars, 1, drain);
+    return;
+  }
+
+  const int g = lane >> 2, t = lane & 3;
+  double *scratch = E + warp * S::S1;
   for (int i = 0;; ++i)
   {
-    const int b    = i & 1;
-    const Item &it = s_item[i % 3];
-    if (it.idx >= q.total)
-      break;
-    if (!it.ok && !q.wait(it, w, tid))
-      break;
-    Item &next     = s_item[(i + 1) % 3];
-    const int part = it.idx % K;
-    q.take(tid);
+    const int b = i & 1;
+    if (!mbar_wait_bounded(&s_bars.full[b], (i >> 1) & 1, drain))
+    {
+      if (lane == 0 && w.status)
+        atomicExch(w.status, 1);
+      return;
+    }
+    const Item &it = s_item[i % ITEM_SLOTS];
+    if (it.idx >= total)
+      return;
+    const int part   = it.idx % K;
     const double *as = stage_a(b);
     // ---- phase 2: this warp's (j_2, j_3) of eight columns, j_1 = warp,
     // columns c = g (on their way during phase 1)
@@ -668,15 +746,18 @@ __global__ void __launch_bounds__(RingMma<N>::THREADS, RingMma<N>::MINB)
     double wv[8][2];
     if (own)
     {
-      const double *wp = static_cast<const double *>(it.ptr[15]) + (long long)warp * N2 * N3 + col;
+      // j_3 = t + 4 s: four consecutive rows of the tile a load
+      const int cw     = min(8, N3 - part * 8);
+      const double *wp = static_cast<const double *>(it.ptr[15]) + part * 8 * N3 +
+                         (warp * N2 + t) * cw + g;
 #pragma unroll
       for (int qq = 0; qq < 8; qq++)
 #pragma unroll
         for (int s = 0; s < 2; s++)
         {
           wv[qq][s] = 0.0;
-          if (N == 8 || (qq < N && 2 * t + s < N && col < N3))
-            wv[qq][s] = w_load(wp + (long long)(qq * N + 2 * t + s) * N3, pol.keep);
+          if (N == 8 || (qq < N && t + 4 * s < N && g < cw))
+            wv[qq][s] = w_load(wp + (qq * N + 4 * s) * cw, pol.keep);
         }
     }
     // ---- phase 1: modes 6, 5, 4 on head row h -> W
@@ -688,43 +769,38 @@ __global__ void __launch_bounds__(RingMma<N>::THREADS, RingMma<N>::MINB)
       frag_of<N>(f.b2, as + 4 * N2, g, t);
       frag_of<N>(f.a3, as + 5 * N2, g, t);
       double v[8][2], acc[8][2];
-      const bool odd = !aligned16(static_cast<const double *>(it.ptr[6]) + (long long)h * N3);
+      const bool odd =
+          !aligned16(static_cast<const double *>(it.ptr[6]) + (long long)part * 8 * N3);
+      const double *row = stage_x(b) + (odd ? 1 : 0) + warp * N3 + g * N + 2 * t;
 #pragma unroll
       for (int qq = 0; qq < 8; qq++)
       {
-        const double *src = row + (odd ? 1 : 0) + qq * N2 + g * N + 2 * t;
         if (N == 8 && !odd)
         {
-          const double2 u = *reinterpret_cast<const double2 *>(src);
+          const double2 u = *reinterpret_cast<const double2 *>(row + qq * N2);
           v[qq][0]        = u.x;
           v[qq][1]        = u.y;
         }
         else
 #pragma unroll
           for (int s = 0; s < 2; s++)
-            v[qq][s] = (N == 8 || (qq < N && g < N && 2 * t + s < N)) ? src[s] : 0.0;
+            v[qq][s] = (N == 8 || (qq < N && g < N && 2 * t + s < N)) ? row[qq * N2 + s] : 0.0;
         acc[qq][0] = acc[qq][1] = 0.0;
       }
       kron8x3_tile<N>(v, acc, f, scratch, g, t);
-      if (tid == 0)
-        q.publish(&next);
-      double *wp = static_cast<double *>(it.ptr[7]) + (long long)h * N3;
+      // W holds tile after tile of eight columns (n = 7: the last has seven),
+      // the head rows of each one after another
+      double *wp = static_cast<double *>(it.ptr[7]);
 #pragma unroll
       for (int qq = 0; qq < N; qq++)
 #pragma unroll
         for (int s = 0; s < 2; s++)
           if (N == 8 || (g < N && 2 * t + s < N))
-            w_store(wp + (2 * t + s) * N2 + qq * N + g, acc[qq][s], pol.keep);
-    }
-    else if (tid == 0)
-      q.publish(&next);
-    // the next item's row and factors
-    __syncwarp(); // the row buffer is read
-    q.mid(w, tid);
-    if (next.idx < q.total)
-    {
-      issue_a(next, b ^ 1);
-      issue_row(next);
+          {
+            const int c  = (2 * t + s) * N2 + qq * N + g;
+            const int cw = N == 8 ? 8 : min(8, N3 - (c & ~7));
+            w_store(wp + (c & ~7) * N3 + h * cw + (c & 7), acc[qq][s], pol.keep);
+          }
     }
     // ---- phase 2, modes 3 and 2
     if (own)
@@ -733,7 +809,9 @@ __global__ void __launch_bounds__(RingMma<N>::THREADS, RingMma<N>::MINB)
 #pragma unroll
       for (int qq = 0; qq < 8; qq++)
         r[qq][0] = r[qq][1] = 0.0;
-      frag_of<N>(b3, as + 2 * N2, g, t);
+#pragma unroll
+      for (int s = 0; s < 2; s++)
+        b3[s] = (N == 8 || (g < N && t + 4 * s < N)) ? as[2 * N2 + g + (t + 4 * s) * N] : 0.0;
       frag_of<N>(b2, as + 1 * N2, g, t);
       mma_along_p(wv, r, b3);
       if (N < 8)
@@ -750,7 +828,7 @@ __global__ void __launch_bounds__(RingMma<N>::THREADS, RingMma<N>::MINB)
         for (int s = 0; s < 2; s++)
           scratch[(2 * t + s) * S::S2 + qq * 8 + g] = r[qq][s];
     }
-    __syncthreads();
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * S::WARPS) : "memory");
     // ---- phase 2, mode 1: warp = i_2
     if (own)
     {
@@ -775,14 +853,12 @@ __global__ void __launch_bounds__(RingMma<N>::THREADS, RingMma<N>::MINB)
           if (N == 8 || (2 * t + s < N && col < N3))
             y_add(y + (long long)((2 * t + s) * N2 + qq) * N3, r[qq][s], pol.stream);
     }
-    q.pub1 = it.slot1;
-    q.pub2 = it.slot2;
-    q.late(s_item[(i + 2) % 3], w, tid);
-    cp_async_wait();
-    __syncthreads();
+    __syncwarp();
+    if (lane == 0)
+      mbar_arrive(&s_bars.done[i % ITEM_SLOTS]);
+    // E is read by every warp before any warp's next transpose
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * S::WARPS) : "memory");
   }
-  if (tid == 0)
-    q.publish(nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -818,8 +894,14 @@ int ring_workspace(const Params &p, const Workspace &wsp, long long L, RingArgs 
   return KRON_SUCCESS;
 }
 
+// Items that each group has between an entry's phases, and again until its slot
+// of W is written anew: a part is published within two items of its being taken
+// (1.6: 3% slower at n = 7; 3: 5% slower at n = 8, whose ring then outgrows the
+// L2 cache).
+constexpr int RING_AHEAD = 2;
+
 template <typename T>
-int ring_launch(const void *fn, int threads, size_t smem, int K, long long L, int ahead, Params p,
+int ring_launch(const void *fn, int threads, int groups, size_t smem, int K, long long L, Params p,
                 const Workspace &wsp, cudaStream_t stream)
 {
   RingArgs w{};
@@ -833,32 +915,32 @@ int ring_launch(const void *fn, int threads, size_t smem, int K, long long L, in
   w.status   = device_status_ptr();
   w.spin     = wait_limit();
   const long long blocks = (long long)device_info().sms * per_sm;
-  // `ahead` items of every block between an entry's phases, and as many until
-  // its slot is written again
-  const int groups = (int)(ahead * blocks / K + 1);
-  w.lag            = std::max(1, std::min({groups, w.nentries, w.slots - 1}));
-  w.slots          = std::min(w.slots, w.lag + groups);
-  w.magic            = (unsigned)(((1ULL << 32) + w.slots - 1) / w.slots);
-  const long long items = (long long)(w.nentries + w.lag) * K;
-  // 32-bit queue positions (two a block taken beyond the end), and the range
+  const int ahead        = (int)(RING_AHEAD * blocks * groups / K + 1); // in entries
+  w.lag                  = std::max(1, std::min({ahead, w.nentries, w.slots - 1}));
+  w.slots                = std::min(w.slots, w.lag + ahead);
+  w.magic                = (unsigned)(((1ULL << 32) + w.slots - 1) / w.slots);
+  const long long items  = (long long)(w.nentries + w.lag) * K;
+  // 32-bit queue positions (one a group taken beyond the end), and the range
   // in which the division by `slots` is exact
   if (items + 3 * blocks > 2147000000LL ||
       ((long long)w.nentries + w.lag) * w.slots >= (1LL << 32))
     return KRON_ERROR_NOT_SUPPORTED;
   ring_init_kernel<T><<<1, 128, 0, stream>>>(w);
-  void *args[] = {&p, &w};
-  return cudaLaunchKernel(fn, dim3((unsigned)std::min(blocks, items)), dim3(threads), args, smem,
-                          stream) == cudaSuccess
+  long long drain      = drain_limit();
+  const long long grid = std::min(blocks, (items + groups - 1) / groups);
+  void *args[]         = {&p, &w, &drain};
+  return cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(threads), args, smem, stream) ==
+                 cudaSuccess
              ? KRON_SUCCESS
              : KRON_ERROR_LAUNCH;
 }
 
-template <typename T, int N, int R, int THREADS, int MINB>
+template <typename T, int N, int R>
 int launch_ring_t(const Params &p, const Workspace &wsp, cudaStream_t stream)
 {
-  using S = RingShape<T, N, R, THREADS>;
-  return ring_launch<T>(reinterpret_cast<const void *>(&kron_ring_kernel<T, N, R, THREADS, MINB>),
-                        THREADS, S::SMEM, S::K, S::L, 2, p, wsp, stream);
+  using S = RingShape<T, N, R>;
+  return ring_launch<T>(reinterpret_cast<const void *>(&kron_ring_kernel<T, N, R>), S::THREADS,
+                        S::GROUPS, S::SMEM, S::K, S::L, p, wsp, stream);
 }
 
 template <int N>
@@ -866,7 +948,7 @@ int launch_ring_mma(const Params &p, const Workspace &wsp, cudaStream_t stream)
 {
   using S = RingMma<N>;
   return ring_launch<double>(reinterpret_cast<const void *>(&kron_ring_mma_kernel<N>), S::THREADS,
-                             S::SMEM, S::K, S::L, 3, p, wsp, stream);
+                             1, S::SMEM, S::K, S::L, p, wsp, stream);
 }
 
 } // namespace
@@ -889,10 +971,10 @@ int launch_ring(const Params &p, int prec, const Workspace &ws, cudaStream_t str
     return KRON_SUCCESS;
   const int n = p.n[0];
   if (prec == PREC_F32)
-    return n == 7   ? launch_ring_t<float, 7, 5, 256, 2>(p, ws, stream)
-           : n == 8 ? launch_ring_t<float, 8, 2, 128, 3>(p, ws, stream)
+    return n == 7   ? launch_ring_t<float, 7, 2>(p, ws, stream)
+           : n == 8 ? launch_ring_t<float, 8, 2>(p, ws, stream)
                     : KRON_ERROR_NOT_SUPPORTED;
-  return n == 6   ? launch_ring_t<double, 6, 3, 128, 3>(p, ws, stream)
+  return n == 6   ? launch_ring_t<double, 6, 3>(p, ws, stream)
          : n == 7 ? launch_ring_mma<7>(p, ws, stream)
                   : launch_ring_mma<8>(p, ws, stream);
 }
