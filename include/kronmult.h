@@ -359,7 +359,11 @@ int kron_l2_persist_reset(kron_stream_t stream);
  *   KRON_VARIANT_MMA8   FP64 tensor-core kernel for d = 3, n = 8
  *   KRON_VARIANT_PIPE   TMA-pipelined passes (n = 3..5, 4-64 KB vectors)
  *   KRON_VARIANT_SQ     on-chip square kernel; param = entries per thread
- *                       block (0: as many as fit)
+ *                       block (0: as many as fit), or KRON_SQ_PACK for
+ *                       several short vectors a warp (n = 2..5, d >= 3, at
+ *                       most 32 fibres of n^2 elements, FP64 and FP32; the
+ *                       built-in choice there, at d = 3, n >= 3 for
+ *                       larger batches)
  *   KRON_VARIANT_GEN    on-chip runtime-shape kernel
  *   KRON_VARIANT_BIG    cluster two-phase kernel; param = cluster size
  *                       (0: default), plus KRON_BIG_CUDA_CORES to keep
@@ -424,6 +428,7 @@ int kron_l2_persist_reset(kron_stream_t stream);
 #define KRON_VARIANT_LARGE 6
 #define KRON_VARIANT_SLAB 7
 #define KRON_VARIANT_SPLIT_TC 8
+#define KRON_SQ_PACK 4096
 #define KRON_BIG_CUDA_CORES 256
 #define KRON_BIG_SMEM_W 512
 #define KRON_BIG_RING 2048

@@ -600,7 +600,11 @@ int launch_variant(Params p, int prec, const Workspace &ws, int variant, int par
     return mma8_supported(p, prec) ? launch_mma8(p, stream) : KRON_ERROR_NOT_SUPPORTED;
   case VAR_PIPE:
     return pipe_supported(p, prec) ? launch_pipe(p, prec, stream) : KRON_ERROR_NOT_SUPPORTED;
+  case VAR_PACK:
+    return pack_supported(p, prec) ? launch_pack(p, prec, stream) : KRON_ERROR_NOT_SUPPORTED;
   case VAR_SQ: {
+    if (param & KRON_SQ_PACK)
+      return launch_variant(p, prec, ws, VAR_PACK, 0, stream);
     if (!is_square(p))
       return KRON_ERROR_NOT_SUPPORTED;
     const int ngmax = sq_entries_max(prec, p.d, p.n[0], merge);
@@ -668,6 +672,7 @@ static bool variant_disabled(int v)
   {
   case VAR_MMA8: return std::getenv("KRON_DISABLE_MMA8") != nullptr;
   case VAR_PIPE: return std::getenv("KRON_DISABLE_PIPE") != nullptr;
+  case VAR_PACK: return std::getenv("KRON_DISABLE_PACK") != nullptr;
   case VAR_RESIDENT: return std::getenv("KRON_DISABLE_RESIDENT") != nullptr;
   case VAR_RING: return std::getenv("KRON_DISABLE_RING") != nullptr;
   case VAR_SLAB: return std::getenv("KRON_DISABLE_SLAB") != nullptr;
@@ -691,6 +696,35 @@ static bool prefer_resident(const Params &p) { return p.eend - p.ebase >= 40; }
 // 60 us).
 static bool prefer_ring(const Params &p) { return p.n[0] > 6 || p.eend - p.ebase >= 192; }
 
+// Packed against square kernel, microseconds.  Most shapes gain at every batch
+// (batched FP64 / FP32, 100000 entries: d = 3, n = 2: 19 / 18 against 31 / 30;
+// d = 4, n = 3: 56 / 43 against 75 / 52; d = 5, n = 3: 133 / 80 against 156 /
+// 97; d = 4, n = 4: 114 / 72 against 171 / 87).  At d = 3, n >= 3 a lane's
+// passes over n^2 elements leave few lanes a warp at work, and the packed
+// form wins with batched vectors only when every warp has several entries (n = 4 FP64
+// 500 / 20000 / 40000 / 100000 entries: 7.9 / 14.6 / 22.8 / 48 against 8.4 /
+// 12.5 / 24.9 / 55; n = 5: 6.4 / 24.8 / 48.5 / 105 against 5.6 / 26.8 / 50.8 /
+// 114; n = 3 FP32: 33.0 against 33.0 at 100000), with shared factors when
+// there is a step of four entries a warp (n = 4, 5: 1600 entries: 6.4, 8.3 against 5.8, 6.0;
+// 8000: 8.4, 10.5 against 9.9, 13.3).  Segmented calls whose groups leave
+// many warps of the last of several turns idle are left out there too (3000 groups: 20.6
+// against 18.7; 1000: 12.1 against 14.5; 4000: 22.8 against 24.8).
+static bool prefer_pack(const Params &p)
+{
+  if (p.d != 3 || p.n[0] < 3)
+    return true;
+  const long long entries = (long long)p.eend - p.ebase;
+  if (p.accum == ACC_DISTINCT)
+    return entries >= 40000;
+  if (p.n[0] == 3)
+    return true;
+  const long long warps = 16LL * device_info().sms; // resident
+  if (!p.seg_off)
+    return entries >= 2 * warps;
+  const long long turns = (p.nitems + warps - 1) / warps;
+  return turns == 1 || 5 * p.nitems >= 4 * turns * warps;
+}
+
 int launch_kron(Params p, int prec, const Workspace &ws, cudaStream_t stream)
 {
   if (p.batch <= 0 || p.eend <= p.ebase)
@@ -712,15 +746,16 @@ int launch_kron(Params p, int prec, const Workspace &ws, cudaStream_t stream)
   // default order: the specialised kernels, then the general ones
   // (VAR_SPLIT_TC: split precision at d = 6, n = 8 on the tcgen05 tensor
   // cores, 3.6 ms for 256 entries against 7.5 ms for the CUDA-core split)
-  // (VAR_RESIDENT and VAR_RING: from the batch on that fills the GPU, see
-  // prefer_resident and prefer_ring; a ring without the workspace for it
+  // (VAR_PACK, VAR_RESIDENT and VAR_RING: where prefer_pack, prefer_resident
+  // and prefer_ring say so; a ring without the workspace for it
   // leaves the call to the next form)
-  static const int order[] = {VAR_MMA8, VAR_PIPE, VAR_RESIDENT, VAR_RING, VAR_SLAB, VAR_SQ,
+  static const int order[] = {VAR_MMA8, VAR_PACK, VAR_PIPE, VAR_RESIDENT, VAR_RING, VAR_SLAB, VAR_SQ,
                               VAR_RECT, VAR_GEN,  VAR_BIG,  VAR_SPLIT_TC, VAR_LARGE};
   const bool env = disable_variables();
   for (int v : order)
   {
-    if ((v == VAR_RESIDENT && !prefer_resident(p)) || (v == VAR_RING && !prefer_ring(p)))
+    if ((v == VAR_RESIDENT && !prefer_resident(p)) || (v == VAR_RING && !prefer_ring(p)) ||
+        (v == VAR_PACK && !prefer_pack(p)))
       continue;
     if (env && variant_disabled(v))
       continue;

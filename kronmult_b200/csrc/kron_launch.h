@@ -34,6 +34,10 @@ int launch_mma8(Params p, cudaStream_t stream);
 bool rect_supported(const Params &p, int prec);
 int launch_rect(const Params &p, cudaStream_t stream);
 
+// Several short vectors a warp, fibres of two modes a lane (kron_pack.cu).
+bool pack_supported(const Params &p, int prec);
+int launch_pack(const Params &p, int prec, cudaStream_t stream);
+
 // TMA-pipelined register-blocked kernel for square n in {2..5}, 4-64 KB
 // vectors (kron_pipe.cu).
 bool pipe_supported(const Params &p, int prec);
@@ -95,6 +99,8 @@ enum Variant : int
   VAR_LARGE = 6, // two-phase launches through the workspace (param unused)
   VAR_SLAB  = 7, // slab-cluster kernel, no workspace; param: KRON_SLAB_NO_ROTATE
   VAR_SPLIT_TC = 8, // split precision d = 6, n = 8 on the tcgen05 tensor cores
+  VAR_PACK = 11,    // several short vectors a warp; in the tuning table it is VAR_SQ with
+                    // KRON_SQ_PACK
   VAR_RECT = 12,    // runtime-shape kernel for whole FP64 vectors (the built-in choice
                     // where VAR_GEN's whole-vector form would run)
   VAR_RESIDENT = 10, // FP32 vector resident in one block; in the tuning table it is
