@@ -154,31 +154,36 @@ __device__ __forceinline__ int entry_index(const Params &p, int e)
   return p.perm ? p.perm[e] : e;
 }
 
-// Balanced contiguous range of positions for group gw of nw (warps, thread
-// groups): positions are split evenly; with output groups (seg_off) the split
-// points snap to the next group start, so that an output group is never
-// shared.
-__device__ __forceinline__ int snap_to_group(const Params &p, long long pos)
+// One round of a search by the warp for the first group s in [lo, hi) with
+// seg_off[s] >= pos: 32 probes, so 8192 groups take three loads in series
+// where a binary search takes thirteen (d = 3, n = 8, 8192 groups of 16: 143.0
+// -> 140.3 us, 3000 of 7: 38.6 -> 37.5; d = 4, n = 3, 100 of 9: 12.3 -> 11.2).
+__device__ __forceinline__ void snap_round(const int *seg_off, long long pos, int &lo, int &hi)
 {
-  int lo = p.ibase, hi = p.ibase + p.nitems; // first s with seg_off[s] >= pos
-  while (lo < hi)
-  {
-    const int mid = (lo + hi) >> 1;
-    if (p.seg_off[mid] < pos)
-      lo = mid + 1;
-    else
-      hi = mid;
-  }
-  return p.seg_off[lo];
+  const long long len = hi - lo;
+  const auto probe    = [&](int i) { return lo + (int)(len * (i + 1) / 33); };
+  const bool below    = len > 0 && seg_off[probe((int)(threadIdx.x & 31))] < pos;
+  const int k         = __popc(__ballot_sync(0xffffffffu, below)); // probes below pos come first
+  const int nlo = k > 0 ? probe(k - 1) + 1 : lo, nhi = k < 32 ? probe(k) : hi;
+  lo            = nlo;
+  hi            = len > 0 ? nhi : lo;
 }
 
+// Balanced contiguous range of positions for group gw of nw (warps, thread
+// groups); an output group (seg_off) is never shared.  Called by whole warps.
 __device__ __forceinline__ void group_range(const Params &p, int gw, int nw, int &eb, int &ee)
 {
   if (p.seg_off)
   {
     const long long b = p.seg_off[p.ibase], tot = p.seg_off[p.ibase + p.nitems] - b;
-    eb = snap_to_group(p, b + tot * gw / nw);
-    ee = snap_to_group(p, b + tot * (gw + 1) / nw);
+    int l0 = p.ibase, h0 = p.ibase + p.nitems, l1 = l0, h1 = h0;
+    while (l0 < h0 || l1 < h1)
+    {
+      snap_round(p.seg_off, b + tot * gw / nw, l0, h0);
+      snap_round(p.seg_off, b + tot * (gw + 1) / nw, l1, h1);
+    }
+    eb = p.seg_off[l0];
+    ee = p.seg_off[l1];
   }
   else
   {

@@ -20,8 +20,15 @@
 // column 2t+1) is absorbed by permuting the rows of the constant A_l^T
 // fragments, so no data moves between modes except the one transpose.
 // Consecutive entries with the same output pointer are summed in the MMA
-// accumulators and written once (atomic red.global.add, or a plain
-// read-modify-write when outputs are exclusive / segmented).
+// accumulators and written once (red.global.add).
+//
+// An entry is about 3600 cycles of a warp for 768 of the tensor pipe, and four
+// warps a pipe keep it 73% busy (131072 entries, 8192 outputs: 123 us).  128
+// registers allow no more warps; bulk copies for x, pointers spread over the
+// lanes, copies between the products or x a step ahead in registers were all
+// slower (129 to 143 us).  Segmented groups stay whole (each output is summed
+// in batch order): 8192 groups of 16 on 2368 warps leave some with 64 entries
+// against 55 on average (140 us).
 #include <cstdint>
 
 #include "kron_launch.h"
