@@ -154,36 +154,71 @@ __device__ __forceinline__ int entry_index(const Params &p, int e)
   return p.perm ? p.perm[e] : e;
 }
 
-// One round of a search by the warp for the first group s in [lo, hi) with
-// seg_off[s] >= pos: 32 probes, so 8192 groups take three loads in series
-// where a binary search takes thirteen (d = 3, n = 8, 8192 groups of 16: 143.0
-// -> 140.3 us, 3000 of 7: 38.6 -> 37.5; d = 4, n = 3, 100 of 9: 12.3 -> 11.2).
-__device__ __forceinline__ void snap_round(const int *seg_off, long long pos, int &lo, int &hi)
+// Search by the warp for the first output group that starts at or behind
+// position pos, of those of [ibase, ibase + nitems]: its start.  The first 32
+// probes lie around `guess`, later rounds split what is left in 33: one or two
+// loads in series where a binary search of 8192 groups takes thirteen
+// (segmented calls: d = 3, n = 8, 8192 groups of 16: 142.7 -> 138.0 us, 2000
+// of 9: 27.3 -> 24.9; d = 4, n = 3, 8000 of 3: 18.7 -> 16.6, 1000 of 3: 8.4 ->
+// 6.0 us).
+struct GroupSearch
 {
-  const long long len = hi - lo;
-  const auto probe    = [&](int i) { return lo + (int)(len * (i + 1) / 33); };
-  const bool below    = len > 0 && seg_off[probe((int)(threadIdx.x & 31))] < pos;
-  const int k         = __popc(__ballot_sync(0xffffffffu, below)); // probes below pos come first
-  const int nlo = k > 0 ? probe(k - 1) + 1 : lo, nhi = k < 32 ? probe(k) : hi;
-  lo            = nlo;
-  hi            = len > 0 ? nhi : lo;
-}
+  int lo, hi, start;
+  bool open;
+  __device__ __forceinline__ void begin(const Params &p, long long pos, int guess)
+  {
+    const int lane = threadIdx.x & 31, end = p.ibase + p.nitems;
+    const int i    = min(max(guess - 16 + lane, p.ibase), end);
+    const int v    = p.seg_off[i];
+    const int k    = __popc(__ballot_sync(0xffffffffu, v < pos)); // those below pos come first
+    start          = __shfl_sync(0xffffffffu, v, k & 31);
+    const int i0   = max(guess - 16, p.ibase);
+    open           = (k == 0 && i0 > p.ibase) || k == 32; // it lies outside the probes
+    lo             = k == 0 ? p.ibase : guess + 16;
+    hi             = k == 0 ? i0 : end;
+  }
+  __device__ __forceinline__ void finish(const Params &p, long long pos)
+  {
+    if (!open)
+      return;
+    while (lo < hi)
+    {
+      const long long len = hi - lo;
+      const auto probe    = [&](int i) { return lo + (int)(len * (i + 1) / 33); };
+      const bool below    = p.seg_off[probe((int)(threadIdx.x & 31))] < pos;
+      const int k         = __popc(__ballot_sync(0xffffffffu, below));
+      const int nlo = k > 0 ? probe(k - 1) + 1 : lo, nhi = k < 32 ? probe(k) : hi;
+      lo            = nlo;
+      hi            = nhi;
+    }
+    start = p.seg_off[lo];
+  }
+};
 
 // Balanced contiguous range of positions for group gw of nw (warps, thread
-// groups); an output group (seg_off) is never shared.  Called by whole warps.
+// groups): positions are split evenly; with output groups (seg_off) the split
+// points snap to the next group start, so that an output group is never
+// shared.  Called by whole warps.
 __device__ __forceinline__ void group_range(const Params &p, int gw, int nw, int &eb, int &ee)
 {
-  if (p.seg_off)
+  if (p.seg_off && p.nitems <= nw) // one at most
+  {
+    const int s = p.ibase + min(gw, p.nitems);
+    eb          = p.seg_off[s];
+    ee          = gw < p.nitems ? p.seg_off[s + 1] : eb;
+  }
+  else if (p.seg_off)
   {
     const long long b = p.seg_off[p.ibase], tot = p.seg_off[p.ibase + p.nitems] - b;
-    int l0 = p.ibase, h0 = p.ibase + p.nitems, l1 = l0, h1 = h0;
-    while (l0 < h0 || l1 < h1)
-    {
-      snap_round(p.seg_off, b + tot * gw / nw, l0, h0);
-      snap_round(p.seg_off, b + tot * (gw + 1) / nw, l1, h1);
-    }
-    eb = p.seg_off[l0];
-    ee = p.seg_off[l1];
+    const long long p0 = b + tot * gw / nw, p1 = b + tot * (gw + 1) / nw;
+    // groups of equal length start there
+    GroupSearch s0, s1;
+    s0.begin(p, p0, p.ibase + (int)((long long)p.nitems * gw / nw));
+    s1.begin(p, p1, p.ibase + (int)((long long)p.nitems * (gw + 1) / nw));
+    s0.finish(p, p0);
+    s1.finish(p, p1);
+    eb = s0.start;
+    ee = s1.start;
   }
   else
   {

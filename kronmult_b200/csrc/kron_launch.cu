@@ -706,9 +706,10 @@ static bool prefer_ring(const Params &p) { return p.n[0] > 6 || p.eend - p.ebase
 // 12.5 / 24.9 / 55; n = 5: 6.4 / 24.8 / 48.5 / 105 against 5.6 / 26.8 / 50.8 /
 // 114; n = 3 FP32: 33.0 against 33.0 at 100000), with shared factors when
 // there is a step of four entries a warp (n = 4, 5: 1600 entries: 6.4, 8.3 against 5.8, 6.0;
-// 8000: 8.4, 10.5 against 9.9, 13.3).  Segmented calls whose groups leave
-// many warps of the last of several turns idle are left out there too (3000 groups: 20.6
-// against 18.7; 1000: 12.1 against 14.5; 4000: 22.8 against 24.8).
+// 8000: 8.4, 10.5 against 9.9, 13.3).  Segmented calls at n = 4, 5 stay with
+// the square kernel whatever their size, since the parts of a call have to
+// sum as the whole does: groups of 8 gain (1000: 10.5 against 14.6), groups of 3
+// lose (4000: 12.5 against 10.5).
 static bool prefer_pack(const Params &p)
 {
   if (p.d != 3 || p.n[0] < 3)
@@ -716,13 +717,7 @@ static bool prefer_pack(const Params &p)
   const long long entries = (long long)p.eend - p.ebase;
   if (p.accum == ACC_DISTINCT)
     return entries >= 40000;
-  if (p.n[0] == 3)
-    return true;
-  const long long warps = 16LL * device_info().sms; // resident
-  if (!p.seg_off)
-    return entries >= 2 * warps;
-  const long long turns = (p.nitems + warps - 1) / warps;
-  return turns == 1 || 5 * p.nitems >= 4 * turns * warps;
+  return p.n[0] == 3 || (!p.seg_off && entries >= 32LL * device_info().sms);
 }
 
 int launch_kron(Params p, int prec, const Workspace &ws, cudaStream_t stream)

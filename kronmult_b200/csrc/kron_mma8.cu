@@ -28,7 +28,7 @@
 // lanes, copies between the products or x a step ahead in registers were all
 // slower (129 to 143 us).  Segmented groups stay whole (each output is summed
 // in batch order): 8192 groups of 16 on 2368 warps leave some with 64 entries
-// against 55 on average (140 us).
+// against 55 on average (138 us).
 #include <cstdint>
 
 #include "kron_launch.h"

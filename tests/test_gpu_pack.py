@@ -116,3 +116,28 @@ def test_builtin_choice_at_d3(gpu_lib, n):
         pY = at(dY, L * yl)
         kb.kronmult_xbatched_segmented(3, n, pA, n, pX, pY, kb.Segments(pY))
         assert rel_err(host(dY), Yref) <= TOL["f64"], groups
+
+
+@pytest.mark.parametrize("groups,hi", [(1, 300), (4000, 2), (4737, 3), (9000, 60), (20001, 2)])
+def test_segment_ranges(gpu_lib, groups, hi):
+    """Groups of very unequal length, so that warps' ranges start far from
+    where equal ones would: fewer groups than warps, and more."""
+    import torch
+
+    d, n, L, npool = 3, 2, 8, 5
+    rng = np.random.default_rng(groups)
+    runs = np.sort(rng.integers(1, hi + 1, groups))
+    runs[groups // 3] = 3000
+    yl = np.repeat(np.arange(groups), runs)
+    batch = len(yl)
+    A, X, Y0 = (rng.uniform(-1, 1, s) for s in (4 * npool, L * 50, L * groups))
+    xl, al = rng.integers(0, 50, batch), rng.integers(0, npool, d * batch)
+    Yref = Y0.copy()
+    oracle.kronmult_general(d, [n] * d, [n] * d, A.ctypes.data + 32 * al, [n] * d,
+                            X.ctypes.data + 8 * L * xl, Yref.ctypes.data + 8 * L * yl)
+    dA, dX, dY = dev(A), dev(X), dev(Y0)
+    at = lambda t, o: t.data_ptr() + 8 * torch.from_numpy(np.asarray(o)).cuda()  # noqa: E731
+    pY = at(dY, L * yl)
+    kb.tune_clear()
+    kb.kronmult_xbatched_segmented(d, n, at(dA, 4 * al), n, at(dX, L * xl), pY, kb.Segments(pY))
+    assert rel_err(host(dY), Yref) <= TOL["f64"]
