@@ -82,7 +82,7 @@ __device__ __forceinline__ void pack_pass(T *x, const T *A, int f)
   for (int c = 0; c < C; c++)
     v[c] = x[S::pos(base + c * ST)];
 #pragma unroll
-  for (int m = k - 1; m >= 0; m--)
+  for (int m = 0; m < k; m++) // in the square kernel's order: the same products, bit for bit
   {
     T A_[S::AF]; // the factor, column major
 #pragma unroll
