@@ -316,25 +316,16 @@ class BatchedSquare(Workload):
         # library's query asks
         need = kb.lib().kron_batched_workspace_bytes(self.d, self.n, self.batch)
         self.dW = torch.empty(max(1, need // 8), dtype=dt, device=dev) if need else None
-        # vectors beyond shared memory: one slab-cluster launch for d=6 n=6
-        # (FP64, FP32), one cluster two-phase launch for d=6 n=7..8 (FP64),
-        # n=7..8 (FP32) and d=5 n=8 (FP64), else the two-phase path's two
-        # launches
+        # vectors beyond shared memory: the ring kernel behind the small one
+        # that clears its control words for d=6 n=7..8 (FP64, FP32) and, from
+        # 192 entries on, n=6 (FP64); one slab-cluster or resident launch for
+        # d=6 n=6 otherwise; one cluster two-phase launch for d=5 n=8 (FP64);
+        # else the two-phase path's two launches
         d, n, prec = self.d, self.n, self.precision
-        if not need:
-            self.launches_per_step = 1
-        elif d == 6 and n == 6 and prec == "f64" and self.batch >= 512:
-            # the slab-cluster kernel and, concurrently on a second stream,
-            # the cluster two-phase kernel on the SMs the slab clusters leave
-            # idle (a share of the entries)
-            self.launches_per_step = 2
-        elif d == 6 and n == 6 and prec in ("f64", "f32"):
-            self.launches_per_step = 1
-        else:
-            fp64 = prec == "f64"
-            cluster = (d == 6 and (6 if fp64 else 7) <= n <= 8 and prec != "split") or \
-                (fp64 and d == 5 and n == 8)
-            self.launches_per_step = 1 if cluster else 2
+        one = not need or (prec == "f64" and d == 5 and n == 8) or \
+            (d == 6 and n == 6 and (prec == "f32" or (prec == "f64" and self.batch < 192))) or \
+            (d == 6 and n >= 7 and prec != "split" and self.batch < 3)
+        self.launches_per_step = 1 if one else 2
         self.e2e_pipeline = (f"{min(E2E_CHUNKS, self.batch)} chunks of entries; uploads, calls "
                              "and downloads overlapped on 3 streams")
         if not e2e:
@@ -680,7 +671,8 @@ class XbatchedBig(Workload):
         self.pX = (self.dX.data_ptr() + 8 * self.L * torch.arange(self.batch)).to(dev)
         self.pY = (self.dY.data_ptr() + 8 * self.L * torch.from_numpy(self.ylist)).to(dev)
         self.pW = (self.dW.data_ptr() + 8 * self.L * torch.arange(self.nw)).to(dev)
-        self.launches_per_step = 1
+        # the ring kernel behind the small one that clears its control words
+        self.launches_per_step = 2
         # e2e host copies: X, Y, A pool and the pointer arrays
         self.h = {k: v.cpu().pin_memory() for k, v in dict(A=self.dA, X=self.dX, Y=self.dY,
                                                           pA=self.pA, pX=self.pX,
@@ -1247,8 +1239,8 @@ def run_ours(args, world, rank, local):
         if tsrc:
             roof["traffic_source"] = tsrc
         if wl.launches_per_step > 1:
-            # achieved and traffic are per launch: the step's bytes over the
-            # step's time (concurrent launches) or each launch's share
+            # achieved is the step's bytes over the step's time; traffic is
+            # the main launch's
             roof["launches_per_step"] = wl.launches_per_step
         line = {"metric": METRIC, "value": round(value, 2), "unit": "GFLOP/s",
                 "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
