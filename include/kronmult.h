@@ -363,7 +363,11 @@ int kron_l2_persist_reset(kron_stream_t stream);
  *                       several short vectors a warp (n = 2..5, d >= 3, at
  *                       most 32 fibres of n^2 elements, FP64 and FP32; the
  *                       built-in choice there, at d = 3, n >= 3 for
- *                       larger batches)
+ *                       larger batches), or KRON_SQ_PAIR for a block an
+ *                       entry and two modes a pass (FP64 and FP32, d = 4..6
+ *                       vectors of 625 to 16807 elements: d = 6, n = 3, 5;
+ *                       d = 5, n = 4..7; d = 4, n = 5..8; the built-in
+ *                       choice for most of them)
  *   KRON_VARIANT_GEN    on-chip runtime-shape kernel
  *   KRON_VARIANT_BIG    cluster two-phase kernel; param = cluster size
  *                       (0: default), plus KRON_BIG_CUDA_CORES to keep
@@ -429,6 +433,7 @@ int kron_l2_persist_reset(kron_stream_t stream);
 #define KRON_VARIANT_SLAB 7
 #define KRON_VARIANT_SPLIT_TC 8
 #define KRON_SQ_PACK 4096
+#define KRON_SQ_PAIR 8192
 #define KRON_BIG_CUDA_CORES 256
 #define KRON_BIG_SMEM_W 512
 #define KRON_BIG_RING 2048

@@ -281,6 +281,7 @@ VARIANTS = {1: "mma8", 2: "pipe", 3: "sq", 4: "gen", 5: "big", 6: "large", 7: "s
             8: "split_tc"}
 # "sq" param: several short vectors a warp (n = 2..5, d >= 3)
 SQ_PACK = 4096
+SQ_PAIR = 8192
 # "big" param bit: FP64 d = 6, n = 8 on CUDA-core FMAs instead of tensor cores
 BIG_CUDA_CORES = 256
 # "big" param bit: keep the intermediate in the cluster's shared memory

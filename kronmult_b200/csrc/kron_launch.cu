@@ -1,5 +1,7 @@
 // Host-side dispatch: picks the kernel family for a problem and launches it.
 //
+//  * square vectors of up to a few KB -> kron_pack_kernel, up to a block's
+//    shared memory -> kron_pair_kernel, where their rules below say so
 //  * square n in 2..8 whose n^d vector (and merge buffer) fits a block's
 //    shared memory            -> kron_sq_kernel<T, d, n>   (compile-time shape)
 //  * any other shape that fits -> kron_rect_kernel (FP64) or kron_gen_kernel<T>
@@ -602,7 +604,11 @@ int launch_variant(Params p, int prec, const Workspace &ws, int variant, int par
     return pipe_supported(p, prec) ? launch_pipe(p, prec, stream) : KRON_ERROR_NOT_SUPPORTED;
   case VAR_PACK:
     return pack_supported(p, prec) ? launch_pack(p, prec, stream) : KRON_ERROR_NOT_SUPPORTED;
+  case VAR_PAIR:
+    return pair_supported(p, prec) ? launch_pair(p, prec, stream) : KRON_ERROR_NOT_SUPPORTED;
   case VAR_SQ: {
+    if (param & KRON_SQ_PAIR)
+      return launch_variant(p, prec, ws, VAR_PAIR, 0, stream);
     if (param & KRON_SQ_PACK)
       return launch_variant(p, prec, ws, VAR_PACK, 0, stream);
     if (!is_square(p))
@@ -673,6 +679,7 @@ static bool variant_disabled(int v)
   case VAR_MMA8: return std::getenv("KRON_DISABLE_MMA8") != nullptr;
   case VAR_PIPE: return std::getenv("KRON_DISABLE_PIPE") != nullptr;
   case VAR_PACK: return std::getenv("KRON_DISABLE_PACK") != nullptr;
+  case VAR_PAIR: return std::getenv("KRON_DISABLE_PAIR") != nullptr;
   case VAR_RESIDENT: return std::getenv("KRON_DISABLE_RESIDENT") != nullptr;
   case VAR_RING: return std::getenv("KRON_DISABLE_RING") != nullptr;
   case VAR_SLAB: return std::getenv("KRON_DISABLE_SLAB") != nullptr;
@@ -720,6 +727,33 @@ static bool prefer_pack(const Params &p)
   return p.n[0] == 3 || (!p.seg_off && entries >= 32LL * device_info().sms);
 }
 
+// Pair kernel against the pipelined and square kernels, microseconds.  Most
+// shapes gain at every batch (FP64 batched: d = 6, n = 3, 10000 entries 47
+// against 132; d = 4, n = 5, 20000: 86 against 258; d = 5, n = 7, 1000: 129
+// against 312; d = 6, n = 5, 1000: 110 against 216).
+// n = 6: with exclusive outputs the square kernel's many warps are the better
+// use of 36 fibres an entry (d = 4, 8000 entries FP64 80 against 73, 600
+// entries 14.3 against 11.3; d = 5, 2000 entries FP64 123 against 121, FP32 72
+// against 55), but for d = 4 in FP32 (8000 entries: 45 against 49).
+// n = 8 and d = 5, n = 4: an entry alone on an SM is faster with 256 threads
+// than with 64 (n = 8 FP64 148 entries 12.3 against 9.2, 300: 16.4 against
+// 20.5; FP32 150: 12.3 against 9.2, 600: 14.3 against 18.4; d = 5, n = 4, 20:
+// 6.1 against 5.4; segmented n = 8, 60 groups of 3: 22.5 against 20.5, 800 of 9:
+// 175 against 324).  Segmented calls may follow the batch there too: the square
+// kernel's sums are the same bit for bit.
+static bool prefer_pair(const Params &p, int prec)
+{
+  const int n = p.n[0];
+  const long long entries = (long long)p.eend - p.ebase, sms = device_info().sms;
+  if (n == 6)
+    return p.accum != ACC_DISTINCT || (p.d == 4 && prec == PREC_F32);
+  if (n == 8) // segmented: a group is worked through in series
+    return (p.seg_off ? p.nitems : entries) > (prec == PREC_F32 ? 2 * sms : sms);
+  if (n == 4)
+    return entries > sms;
+  return true;
+}
+
 int launch_kron(Params p, int prec, const Workspace &ws, cudaStream_t stream)
 {
   if (p.batch <= 0 || p.eend <= p.ebase)
@@ -741,16 +775,16 @@ int launch_kron(Params p, int prec, const Workspace &ws, cudaStream_t stream)
   // default order: the specialised kernels, then the general ones
   // (VAR_SPLIT_TC: split precision at d = 6, n = 8 on the tcgen05 tensor
   // cores, 3.6 ms for 256 entries against 7.5 ms for the CUDA-core split)
-  // (VAR_PACK, VAR_RESIDENT and VAR_RING: where prefer_pack, prefer_resident
-  // and prefer_ring say so; a ring without the workspace for it
+  // (VAR_PACK, VAR_PAIR, VAR_RESIDENT and VAR_RING: where prefer_pack,
+  // prefer_pair, prefer_resident and prefer_ring say so; a ring without the workspace for it
   // leaves the call to the next form)
-  static const int order[] = {VAR_MMA8, VAR_PACK, VAR_PIPE, VAR_RESIDENT, VAR_RING, VAR_SLAB, VAR_SQ,
+  static const int order[] = {VAR_MMA8, VAR_PACK, VAR_PAIR, VAR_PIPE, VAR_RESIDENT, VAR_RING, VAR_SLAB, VAR_SQ,
                               VAR_RECT, VAR_GEN,  VAR_BIG,  VAR_SPLIT_TC, VAR_LARGE};
   const bool env = disable_variables();
   for (int v : order)
   {
     if ((v == VAR_RESIDENT && !prefer_resident(p)) || (v == VAR_RING && !prefer_ring(p)) ||
-        (v == VAR_PACK && !prefer_pack(p)))
+        (v == VAR_PACK && !prefer_pack(p)) || (v == VAR_PAIR && !prefer_pair(p, prec)))
       continue;
     if (env && variant_disabled(v))
       continue;

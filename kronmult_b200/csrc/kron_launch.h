@@ -38,6 +38,11 @@ int launch_rect(const Params &p, cudaStream_t stream);
 bool pack_supported(const Params &p, int prec);
 int launch_pack(const Params &p, int prec, cudaStream_t stream);
 
+// Mid-size square vectors, a block an entry, fibres of two modes a thread
+// (kron_pair.cu).
+bool pair_supported(const Params &p, int prec);
+int launch_pair(const Params &p, int prec, cudaStream_t stream);
+
 // TMA-pipelined register-blocked kernel for square n in {2..5}, 4-64 KB
 // vectors (kron_pipe.cu).
 bool pipe_supported(const Params &p, int prec);
@@ -101,6 +106,8 @@ enum Variant : int
   VAR_SPLIT_TC = 8, // split precision d = 6, n = 8 on the tcgen05 tensor cores
   VAR_PACK = 11,    // several short vectors a warp; in the tuning table it is VAR_SQ with
                     // KRON_SQ_PACK
+  VAR_PAIR = 13,    // a block an entry, two modes a pass; in the tuning table it is VAR_SQ
+                    // with KRON_SQ_PAIR
   VAR_RECT = 12,    // runtime-shape kernel for whole FP64 vectors (the built-in choice
                     // where VAR_GEN's whole-vector form would run)
   VAR_RESIDENT = 10, // FP32 vector resident in one block; in the tuning table it is

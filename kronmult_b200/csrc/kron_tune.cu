@@ -198,6 +198,7 @@ extern "C" int kron_autotune(int d, int n, int precision, int batch, int *varian
   std::vector<std::pair<int, int>> cand = {
       {VAR_MMA8, 0}, {VAR_PIPE, 0}, {VAR_SLAB, KRON_SLAB_RESIDENT}, {VAR_SLAB, 0}};
   cand.push_back({VAR_SQ, KRON_SQ_PACK});
+  cand.push_back({VAR_SQ, KRON_SQ_PAIR});
   const int ngmax = sq_entries_max(precision, d, n, false);
   for (int ng = 1; ng <= ngmax; ng *= 2)
     cand.push_back({VAR_SQ, ng});
