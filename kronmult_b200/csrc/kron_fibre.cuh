@@ -1,7 +1,7 @@
 // Register-blocked fibres of two modes: an n x n block of a vector held by one
 // thread, v[a n + b], with b the faster mode, and the products of it with one
-// n x n factor along either mode.  Shared by the slab-cluster kernel and the
-// ring kernel.
+// n x n factor along either mode.  Shared by the slab-cluster, resident, ring
+// and pair kernels.
 #pragma once
 
 #include <type_traits>
