@@ -25,8 +25,8 @@
 // through a load, an add and a store: an FP32 add in the L2 cache would flush
 // subnormals.
 //
-// Bound by shared memory and FP64 issue with two to seven warps a block, no
-// longer by exposed latency: batched FP64, before and after, d = 4, n = 8, 6000
+// Bound by latency with few warps an SM (n = 8: six, by shared memory and
+// registers; an instruction in 26% of a scheduler's cycles): batched FP64, before and after, d = 4, n = 8, 6000
 // entries 324 -> 165 us (0.60 GB, HBM alone 92); d = 5, n = 7, 1000 entries 312
 // -> 129 (62); d = 6, n = 3, 10000 entries 132 -> 47 (27); 7200 entries of d = 4,
 // n = 8 on 800 outputs 332 -> 163; 36000 of d = 4, n = 5 on 4000 360 -> 89.

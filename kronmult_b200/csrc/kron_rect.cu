@@ -13,8 +13,10 @@
 // (kronmult_vbatched.hpp:17-228 copies x to scratch and runs one 64-thread
 // block per entry through global memory.)
 //
-// 4096 entries of 576 elements (60 MB): 94 -> 33 us, of which HBM alone would
-// take 9; the instructions of the steps are the bound now.  Before, two
+// 4096 entries of 576 elements (60 MB): 94 -> 30 us, of which HBM alone would
+// take 9; fifteen warps an SM that wait for the steps' latencies are the bound
+// now (an instruction in 34% of a scheduler's cycles, the shared-memory pipe
+// 31% busy).  Before, two
 // groups a block worked through runs of eight entries in series, recomputing
 // every step's shape, dividing per fibre, and waiting out each load.
 #include <algorithm>
@@ -135,7 +137,7 @@ __global__ void __launch_bounds__(RECT_THREADS, MINB)
     }
     // the vector's stage is one of the two buffers, the third the other
     double *cur = base + b * r.buf, *nxt = base + 2 * r.buf;
-    rect_modes<double, AREG>(r.st, d, 1, cur, nxt, base + 3 * r.buf + b * ((r.asz + 1) & ~1), t, GS, g);
+    rect_modes<double, AREG, true>(r.st, d, 1, cur, nxt, base + 3 * r.buf + b * ((r.asz + 1) & ~1), t, GS, g);
     double *y = const_cast<double *>(s_ptr[g][i % 3][7]);
     for (int q = t; q < r.nout; q += GS)
       red_add(y + q, cur[q]);

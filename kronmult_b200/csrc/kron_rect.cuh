@@ -90,6 +90,36 @@ __device__ __forceinline__ void rect_fibres(const T *cur, T *nxt, const T *A, in
   }
 }
 
+// The innermost mode (inner = 1), a thread an output element: fibres a thread
+// apart would be read at a stride of NQ elements and written at one of MQ, up to
+// eight bank passes an access.  Here the threads of a fibre read the same element
+// and writes are contiguous; a thread keeps its row of the factor, NQ elements.
+// (Threads beyond a whole number of fibres have no work.)  4096 entries of 576
+// elements: 32.8 -> 30.5 us; uneven plans, whose items hold many more fibres,
+// lose 0.4% and keep the fibres.
+template <typename T, int NQ, int MQ>
+__device__ __forceinline__ void rect_innermost(const T *cur, T *nxt, const T *A, int nfib, int t,
+                                               int GS)
+{
+  const int per = GS / MQ; // fibres a round
+  const int o0 = t / MQ, i = t - o0 * MQ;
+  if (o0 >= per || o0 >= nfib)
+    return;
+  T a[NQ];
+#pragma unroll
+  for (int j = 0; j < NQ; j++)
+    a[j] = A[i + j * MQ];
+  for (int o = o0; o < nfib; o += per)
+  {
+    const T *src = cur + o * NQ;
+    T z          = T(0);
+#pragma unroll
+    for (int j = 0; j < NQ; j++)
+      z = fma(a[j], src[j], z);
+    nxt[o * MQ + i] = z;
+  }
+}
+
 // Sizes beyond 8: one output element at a time (rare shapes, kept simple).
 template <typename T>
 __device__ __noinline__ void rect_step_any(const T *cur, T *nxt, const T *A, int nq, int mq,
@@ -111,7 +141,7 @@ __device__ __noinline__ void rect_step_any(const T *cur, T *nxt, const T *A, int
 }
 
 // all steps over `rows` consecutive vectors; cur holds the result at the end
-template <typename T, int AREG_MAX>
+template <typename T, int AREG_MAX, bool BY_OUTPUT = false>
 __device__ __forceinline__ void rect_modes(const RectStep *st, int ns, int rows, T *&cur, T *&nxt,
                                            const T *As, int t, int GS, int g)
 {
@@ -123,7 +153,10 @@ __device__ __forceinline__ void rect_modes(const RectStep *st, int ns, int rows,
     {
 #define KRON_RM(NQ_, MQ_)                                                                       \
   case NQ_ * 16 + MQ_:                                                                          \
-    rect_fibres<T, AREG_MAX, NQ_, MQ_>(cur, nxt, As, inner, q.magic, nfib, t, GS);                        \
+    if (BY_OUTPUT && MQ_ > 1 && inner == 1)                                                     \
+      rect_innermost<T, NQ_, MQ_>(cur, nxt, As, nfib, t, GS);                                   \
+    else                                                                                        \
+      rect_fibres<T, AREG_MAX, NQ_, MQ_>(cur, nxt, As, inner, q.magic, nfib, t, GS);            \
     break;
 #define KRON_RM_ROW(NQ_)                                                                        \
   KRON_RM(NQ_, 1) KRON_RM(NQ_, 2) KRON_RM(NQ_, 3) KRON_RM(NQ_, 4) KRON_RM(NQ_, 5)              \
