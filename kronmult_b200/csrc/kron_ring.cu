@@ -21,16 +21,17 @@
 //
 // The control words (queue, abort, and per slot the parts done of each phase,
 // counted up over the slot's generations) lie in the workspace vector after
-// the ring, zeroed by a small kernel ahead of this one.  Waits are bounded (wait_limit() polls): a block that
-// gives up records 1 in the device status word, raises the abort word, which
-// ends the others' waits, and leaves; y of the parts not done is untouched.
+// the ring, zeroed by a small kernel ahead of this one.  Waits are bounded
+// (wait_limit() polls): a group that gives up records 1 in the device status
+// word, raises the abort word, which ends the others' waits, and leaves as a
+// whole once its copies have landed; y of the parts not done is untouched.
 //
 // Measured against what ran before (the cluster two-phase kernel, whose W
 // goes through HBM and back: 9.35 against 6.9 GB for 1024 entries of n = 8;
 // n = 6: the slab-cluster kernel with its side kernel):
-//   n = 6, 4096 entries  1.40 -> 1.23 ms (HBM alone 0.70)
-//   n = 7, 256 entries   0.465 -> 0.243 ms (HBM alone 0.11)
-//   n = 8, 1024 entries with aliasing outputs  2.05 -> 1.70 ms (FP64 tensor
+//   n = 6, 4096 entries  1.40 -> 1.17 ms (HBM alone 0.70)
+//   n = 7, 256 entries   0.465 -> 0.241 ms (HBM alone 0.11)
+//   n = 8, 1024 entries with aliasing outputs  2.05 -> 1.71 ms (FP64 tensor
 //   pipe alone 0.70, HBM 0.98)
 #include <algorithm>
 #include <cstdint>
@@ -218,12 +219,18 @@ __device__ __forceinline__ void item_plan(Item &it, int idx, int total, const Ri
 //            taker in their place, for the end of the queue);
 //   read[d]  the publisher has read description d.
 // (No barrier can run two phases ahead of a thread that waits for it.)
-// All waits are bounded; when one runs out, the status and abort words are
-// raised and the computing warps find the end of the queue.
+// All waits are bounded.  When one of the taker's runs out, it raises the status
+// and abort words and the computing warps find the end of the queue.  When one
+// of the computing warps' does, that warp raises them and `left`, and the group's
+// warps leave together at the item's barrier, which carries their vote (a warp
+// that left alone would leave the others at the barrier for ever); `left` ends
+// the waits of the taker and the publisher for them.  Who leaves early first lets
+// the copies that it waits for or started land.
 constexpr int ITEM_SLOTS = 4;
 struct ControlBars
 {
   uint64_t full[2], done[ITEM_SLOTS], read[ITEM_SLOTS];
+  int left; // the computing warps have given up
 };
 
 // one thread, before the block's first barrier; `warps` that compute
@@ -236,6 +243,26 @@ __device__ __forceinline__ void control_init(ControlBars &bars, int warps)
     mbar_init(&bars.done[d], warps);
     mbar_init(&bars.read[d], 1);
   }
+  bars.left = 0;
+}
+
+// the group's computing warps have left, or are about to
+__device__ __forceinline__ bool has_left(const ControlBars &bars)
+{
+  return *reinterpret_cast<const volatile int *>(&bars.left) != 0;
+}
+
+// A barrier of THREADS threads (whole warps) that ANDs what they bring.
+template <int THREADS>
+__device__ __forceinline__ bool vote_sync(int id, bool v)
+{
+  int all;
+  asm volatile("{\n .reg .pred p, q;\n setp.ne.s32 p, %1, 0;\n"
+               " bar.red.and.pred q, %2, %3, p;\n selp.s32 %0, 1, 0, q;\n}"
+               : "=r"(all)
+               : "r"((int)v), "r"(id), "n"(THREADS)
+               : "memory");
+  return all != 0;
 }
 
 // a bulk copy of this lane's that full[s] waits for
@@ -259,6 +286,43 @@ __device__ __forceinline__ void mbar_arrive(uint64_t *bar)
 template <typename T, int K>
 struct RingControl
 {
+  // one thread
+  static __device__ __forceinline__ void raise(const RingArgs &w)
+  {
+    if (w.status)
+      atomicExch(w.status, 1);
+    atomicExch(ring_ctl<T>(w) + CTL_ABORT, 1);
+  }
+
+  // one thread: the copies of item j, whose mbarrier has its arrivals, land
+  static __device__ __forceinline__ void land(ControlBars &bars, int j, long long drain)
+  {
+    mbar_wait_bounded(&bars.full[j & 1], (j >> 1) & 1, drain);
+  }
+
+  // a computing warp whose wait for item i has run out, ahead of the vote
+  static __device__ __forceinline__ void leave(const RingArgs &w, ControlBars &bars, int i,
+                                            long long drain)
+  {
+    raise(w);
+    *reinterpret_cast<volatile int *>(&bars.left) = 1;
+    land(bars, i, drain);
+  }
+
+  // a wait for the computing warps, over when those have left
+  static __device__ __forceinline__ bool wait_alive(uint64_t *bar, unsigned parity,
+                                                    const ControlBars &bars, long long limit)
+  {
+    for (long long polls = 0; polls < limit; polls++)
+    {
+      if (mbar_try_wait(bar, parity))
+        return true;
+      if (has_left(bars))
+        return false;
+    }
+    return false;
+  }
+
   // one warp, beside `warps` that compute; issue(item, slot, full) starts the
   // copies of an item (whole warp)
   template <typename Issue>
@@ -309,13 +373,28 @@ struct RingControl
       Item &it      = items[j % D];
       uint64_t *bar = &bars.full[j & 1];
       const int idx = __shfl_sync(FULL, q, 0);
-      bool ok       = (j < 2 || mbar_wait_bounded(&bars.done[(j - 2) % D], ((j - 2) / D) & 1, drain)) &&
+      bool ok       = (j < 2 || wait_alive(&bars.done[(j - 2) % D], ((j - 2) / D) & 1, bars, drain)) &&
                 (j < D || mbar_wait_bounded(&bars.read[j % D], (j / D - 1) & 1, drain));
       ok = __all_sync(FULL, ok);
+      if (!ok)
+      {
+        // nothing of this item was started, and the mbarrier it would use may
+        // still be that of item j - 2; computing warps that have not left run
+        // into their bound
+        if (lane == 0)
+        {
+          raise(w);
+          if (j > 1)
+            land(bars, j - 2, drain);
+          if (j > 0)
+            land(bars, j - 1, drain);
+        }
+        return;
+      }
       if (lane == 0 && idx < total)
         q = atomicAdd(ctl + CTL_QUEUE, 1);
       if (lane == 0)
-        item_plan<K>(it, ok ? idx : total, total, w);
+        item_plan<K>(it, idx, total, w);
       if (lane < 16)
       {
         int g         = idx / K - (lane < 8 ? 0 : w.lag);
@@ -333,7 +412,7 @@ struct RingControl
       // the slot's last readers come before the copies
       fence_proxy_async();
       __syncwarp();
-      const bool end = !ok || idx >= total;
+      const bool end = idx >= total;
       if (!end)
         issue(it, j & 1, bar);
       asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_addr(bar))
@@ -355,18 +434,10 @@ struct RingControl
         }
         __threadfence(); // what the others published is visible from here on
       }
-      if (!ok || !met)
+      if (!met && lane == 0)
       {
-        // the copies land in a buffer that nobody reads any more
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncwarp();
-        if (lane == 0)
-        {
-          if (w.status)
-            atomicExch(w.status, 1);
-          atomicExch(ctl + CTL_ABORT, 1);
-          it.idx = total;
-        }
+        raise(w);
+        it.idx = total;
       }
       if (lane == 0)
         mbar_arrive(bar);
@@ -376,18 +447,21 @@ struct RingControl
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(&bars.done[j % D])),
                        "r"(warps)
                        : "memory");
+        if (!met && lane == 0) // computing warps that have left wait for no copy of this item
+          land(bars, j, drain);
         return;
       }
     }
   }
 
   // One thread: publishes the parts of item j of a group once its computing
-  // warps are done with it.  0: not yet, 1: published, -1: the end of the queue.
+  // warps are done with it.  0: not yet, 1: published, -1: the end of the queue,
+  // or they have left without it.
   static __device__ __forceinline__ int publish(const RingArgs &w, const Item *items,
                                                 ControlBars &bars, int j, int total)
   {
     if (!mbar_try_wait(&bars.done[j % ITEM_SLOTS], (j / ITEM_SLOTS) & 1))
-      return 0;
+      return has_left(bars) ? -1 : 0;
     const Item &it = items[j % ITEM_SLOTS];
     if (it.idx >= total)
       return -1;
@@ -559,21 +633,17 @@ __global__ void __launch_bounds__(RingShape<T, N, R>::THREADS, 1)
   ControlBars &bars = s_bars[gr];
   for (int i = 0;; ++i)
   {
-    const int b = i & 1;
-    if (!mbar_wait_bounded(&bars.full[b], (i >> 1) & 1, drain))
-    {
-      if (lane == 0 && w.status)
-        atomicExch(w.status, 1);
-      return;
-    }
+    const int b    = i & 1;
     const Item &it = items[i % ITEM_SLOTS];
-    if (it.idx >= total)
-      return;
+    const bool ok  = __all_sync(0xffffffffu, mbar_wait_bounded(&bars.full[b], (i >> 1) & 1, w.spin));
+    if (!ok && lane == 0)
+      RingControl<T, K>::leave(w, bars, i, drain);
+    const bool go  = ok && it.idx < total;
     const int part = it.idx % K;
     const T *as    = stage_a(gr, b);
     // ---- phase 1, modes 5 and 6 in place
     const int h0   = part * R;
-    const int nfib = it.slot1 >= 0 ? min(R, LH - h0) * N2 : 0;
+    const int nfib = go && it.slot1 >= 0 ? min(R, LH - h0) * N2 : 0;
     T *xs          = stage_a(gr, b) + S::ASZ;
     if constexpr (!S::VEC)
       if (nfib > 0)
@@ -588,7 +658,8 @@ __global__ void __launch_bounds__(RingShape<T, N, R>::THREADS, 1)
       apply_slow<T, N>(v, as + 4 * N2);
       store_chunk<T, N>(c, v);
     }
-    asm volatile("bar.sync %0, 128;" ::"r"(gr + 1) : "memory");
+    if (!vote_sync<S::G>(gr + 1, go)) // the end of the queue, or a wait that ran out
+      return;
     // ---- phase 1, modes 3 and 4; results into W
     if (tid < nfib)
     {
@@ -727,22 +798,18 @@ __global__ void __launch_bounds__(RingMma<N>::THREADS, RingMma<N>::MINB)
   double *scratch = E + warp * S::S1;
   for (int i = 0;; ++i)
   {
-    const int b = i & 1;
-    if (!mbar_wait_bounded(&s_bars.full[b], (i >> 1) & 1, drain))
-    {
-      if (lane == 0 && w.status)
-        atomicExch(w.status, 1);
-      return;
-    }
+    const int b    = i & 1;
     const Item &it = s_item[i % ITEM_SLOTS];
-    if (it.idx >= total)
-      return;
+    const bool ok  = __all_sync(0xffffffffu, mbar_wait_bounded(&s_bars.full[b], (i >> 1) & 1, w.spin));
+    if (!ok && lane == 0)
+      RingControl<double, K>::leave(w, s_bars, i, drain);
+    const bool go    = ok && it.idx < total;
     const int part   = it.idx % K;
     const double *as = stage_a(b);
     // ---- phase 2: this warp's (j_2, j_3) of eight columns, j_1 = warp,
     // columns c = g (on their way during phase 1)
     const int col  = part * 8 + g;
-    const bool own = it.slot2 >= 0 && warp < N;
+    const bool own = go && it.slot2 >= 0 && warp < N;
     double wv[8][2];
     if (own)
     {
@@ -762,7 +829,7 @@ __global__ void __launch_bounds__(RingMma<N>::THREADS, RingMma<N>::MINB)
     }
     // ---- phase 1: modes 6, 5, 4 on head row h -> W
     const int h = part * 8 + warp;
-    if (it.slot1 >= 0 && h < N3)
+    if (go && it.slot1 >= 0 && h < N3)
     {
       AFrag8 f;
       frag_of<N>(f.b1, as + 3 * N2, g, t);
@@ -828,7 +895,8 @@ __global__ void __launch_bounds__(RingMma<N>::THREADS, RingMma<N>::MINB)
         for (int s = 0; s < 2; s++)
           scratch[(2 * t + s) * S::S2 + qq * 8 + g] = r[qq][s];
     }
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * S::WARPS) : "memory");
+    if (!vote_sync<32 * S::WARPS>(1, go)) // the end of the queue, or a wait that ran out
+      return;
     // ---- phase 2, mode 1: warp = i_2
     if (own)
     {
