@@ -106,7 +106,7 @@ struct VParams
   const double *const *pX;
   double *const *pY;
   double *ws;                 // huge class: per-entry regions
-  int budget;                 // shared elements per block
+  int budget;                 // shared elements per block, BUF_SLACK among them
 };
 
 // 8-byte global -> shared copy through the LSU's asynchronous path
@@ -522,7 +522,7 @@ struct kron_vplan_st
   int *d_counters;            // NCOUNT work counters + one chunk counter per huge entry
   double flops;
   size_t ws_bytes;
-  int budget;                 // shared elements per block
+  int budget;                 // shared elements per block, BUF_SLACK among them
   int grid_work;              // work units of the launch (grid upper bound)
   // graph cache
   cudaGraphExec_t exec;
@@ -597,6 +597,10 @@ void sort_by_cost(std::vector<Ranked> &v)
   }
 }
 
+// Elements beyond an entry's budget that its buffers may take: two a buffer,
+// where x starts at the offset it has in a 16-byte unit, and a chunk's odd rows.
+constexpr int BUF_SLACK = 6;
+
 // Two-phase split of a huge entry for a block of `budget` shared elements:
 // phase 1 applies modes [q, d) to chunks of R head rows, phase 2 modes
 // [0, q) to column tiles of C columns.  Prefers tiles of >= 16 columns
@@ -628,7 +632,7 @@ bool plan_huge(int d, const int *m, const int *n, long long budget, HugeSplit &b
       a1 += (long long)m[l] * n[l];
       Mtail *= m[l];
     }
-    const long long R = (budget - even(a1) - 8) / (2 * r1);
+    const long long R = (budget - even(a1) - 2) / (2 * r1);
     const long long C = std::min<long long>({255, Mtail, (budget - even(a2) - 2) / (2 * r2)});
     if (R < 1 || C < 1)
       continue;
@@ -655,10 +659,14 @@ extern "C" int kron_vplan_create(kron_vplan_t *plan, int batchCount, int const s
   *plan = nullptr;
   const DeviceInfo &di = device_info();
   // shared elements per block: two blocks per SM (1 KB of each block's share
-  // is reserved by the hardware; 4 KB cover the kernel's own variables)
-  const long long budget =
+  // is reserved by the hardware; 4 KB cover the kernel's own variables and the
+  // slack).  A plan with a shape that only 2 KB more can hold (a factor of 118 x
+  // 118) runs one block per SM.
+  const long long two_blocks =
       (std::min<long long>(di.max_smem_optin, di.smem_per_sm / VP_MINB - 1024) - 4096) / 8 & ~1LL;
-  static_assert(sizeof(NextSlot) * 2 * VP_WARPS + 64 <= 4096, "the kernel's own variables");
+  static_assert(sizeof(NextSlot) * 2 * VP_WARPS + 8 * BUF_SLACK + 64 <= 4096,
+                "the kernel's own variables");
+  long long budget = two_blocks;
   // class and cost of every entry, then descriptors and steps in queue order
   std::vector<Ranked> cls[NCLS];
   std::vector<HugeSplit> splits; // of the huge entries, in entry order
@@ -674,43 +682,58 @@ extern "C" int kron_vplan_create(kron_vplan_t *plan, int batchCount, int const s
     }
     return s[0];
   };
-  for (int k = 0; k < batchCount; k++)
+  auto classify = [&]() {
+    for (int k = 0; k < batchCount; k++)
+    {
+      const int d = shapes[13LL * k];
+      if (d < 1 || d > MAXD)
+        return (int)KRON_ERROR_INVALID_VALUE;
+      shape_of(k);
+      long long asz = 0;
+      for (int l = 0; l < d; l++)
+      {
+        if (m[l] < 1 || n[l] < 1 || m[l] > 255 || n[l] > 255)
+          return (int)KRON_ERROR_INVALID_VALUE;
+        asz += (long long)m[l] * n[l];
+      }
+      const OrderCost oc = order_cost(d, m, n);
+      total_flops += oc.flops;
+      const long long mi   = even(oc.elems) + 2;
+      const long long need = 2 * mi + even(asz);
+      int c;
+      if (mi <= WARP_MAX && need <= (budget / VP_WARPS & ~1LL))
+        c = CLS_WARP;
+      else if (need <= (budget / 4 & ~1LL))
+        c = CLS_QUAD;
+      else if (need <= (budget / 2 & ~1LL))
+        c = CLS_HALF;
+      else if (need <= budget + 4) // with the four elements of x's offsets
+        c = CLS_BLOCK;
+      else
+      {
+        c = CLS_HUGE;
+        HugeSplit hs;
+        if (!plan_huge(d, m, n, budget, hs))
+          return (int)KRON_ERROR_NOT_SUPPORTED;
+        split_of[k] = (int)splits.size();
+        splits.push_back(hs);
+      }
+      cls[c].push_back(Ranked{(float)oc.flops, k});
+    }
+    return (int)KRON_SUCCESS;
+  };
+  int rc = classify();
+  if (rc == KRON_ERROR_NOT_SUPPORTED)
   {
-    const int d = shapes[13LL * k];
-    if (d < 1 || d > MAXD)
-      return KRON_ERROR_INVALID_VALUE;
-    shape_of(k);
-    long long asz = 0;
-    for (int l = 0; l < d; l++)
-    {
-      if (m[l] < 1 || n[l] < 1 || m[l] > 255 || n[l] > 255)
-        return KRON_ERROR_INVALID_VALUE;
-      asz += (long long)m[l] * n[l];
-    }
-    const OrderCost oc = order_cost(d, m, n);
-    total_flops += oc.flops;
-    const long long mi   = even(oc.elems) + 2;
-    const long long need = 2 * mi + even(asz);
-    int c;
-    if (mi <= WARP_MAX && need <= (budget / VP_WARPS & ~1LL))
-      c = CLS_WARP;
-    else if (need <= (budget / 4 & ~1LL))
-      c = CLS_QUAD;
-    else if (need <= (budget / 2 & ~1LL))
-      c = CLS_HALF;
-    else if (need <= budget)
-      c = CLS_BLOCK;
-    else
-    {
-      c = CLS_HUGE;
-      HugeSplit hs;
-      if (!plan_huge(d, m, n, budget, hs))
-        return KRON_ERROR_NOT_SUPPORTED;
-      split_of[k] = (int)splits.size();
-      splits.push_back(hs);
-    }
-    cls[c].push_back(Ranked{(float)oc.flops, k});
+    budget = two_blocks + 256;
+    for (auto &c : cls)
+      c.clear();
+    splits.clear();
+    total_flops = 0.0;
+    rc          = classify();
   }
+  if (rc != KRON_SUCCESS)
+    return rc;
   kron_vplan_st *pl = new (std::nothrow) kron_vplan_st();
   if (!pl)
     return KRON_ERROR_ALLOC;
@@ -816,7 +839,7 @@ extern "C" int kron_vplan_create(kron_vplan_t *plan, int batchCount, int const s
 
   pl->nitems     = (int)items.size();
   pl->flops      = total_flops;
-  pl->budget     = (int)budget;
+  pl->budget     = (int)budget + BUF_SLACK;
   pl->ws_bytes   = (size_t)woff * 8;
   pl->grid_work  = (int)std::min<long long>(
       1LL << 30, (long long)items.size() + pl->nblock + (pl->nhalf + 1) / 2 +
