@@ -32,7 +32,7 @@ namespace {
 
 using namespace ptx;
 
-constexpr int RECT_THREADS = 256;
+constexpr int RECT_THREADS = 256, RECT_WIDE = 512;
 
 struct RectArgs
 {
@@ -50,14 +50,14 @@ __device__ __forceinline__ void cp8(double *dst, const double *src)
 }
 
 // AREG, MINB: elements of a factor held in registers, blocks per SM
-template <int AREG, int MINB>
-__global__ void __launch_bounds__(RECT_THREADS, MINB)
+template <int THREADS, int AREG, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB)
     kron_rect_kernel(const __grid_constant__ Params p, const __grid_constant__ RectArgs r)
 {
   extern __shared__ __align__(16) double smem[];
   __shared__ const double *s_ptr[8][3][8]; // per group: pointers of three entries
   const int GS = r.GS;
-  const int ng = RECT_THREADS / GS, g = threadIdx.x / GS, t = threadIdx.x - g * GS;
+  const int ng = THREADS / GS, g = threadIdx.x / GS, t = threadIdx.x - g * GS;
   double *base = smem + (size_t)g * r.group;
   int e, ee;
   group_range(p, blockIdx.x * ng + g, gridDim.x * ng, e, ee);
@@ -207,25 +207,37 @@ int launch_rect(const Params &p, cudaStream_t stream)
   // registers (80 a thread); longer ones reuse a factor over more fibres and
   // gain from holding up to 36 (two blocks; 576 elements: 31 against 35 us,
   // 96 elements: 42 against 50 us the other way)
-  const void *fn = r.buf < 512 ? reinterpret_cast<const void *>(&kron_rect_kernel<16, 3>)
-                               : reinterpret_cast<const void *>(&kron_rect_kernel<36, 2>);
-  // as many groups a block as its threads and the shared memory give
-  const int maxsm = device_info().max_smem_optin - 2048;
-  while (r.GS < RECT_THREADS && (long long)(RECT_THREADS / r.GS) * r.group * 8 > maxsm)
-    r.GS *= 2;
-  if ((long long)(RECT_THREADS / r.GS) * r.group * 8 > maxsm)
+  const void *fn = r.buf < 512
+                       ? reinterpret_cast<const void *>(&kron_rect_kernel<RECT_THREADS, 16, 3>)
+                       : reinterpret_cast<const void *>(&kron_rect_kernel<RECT_THREADS, 36, 2>);
+  // as many groups a block as its threads and half an SM's shared memory give
+  // (1 KB a block is the hardware's, 2 KB hold the kernel's own variables), at
+  // least one: groups twice as large are faster than one block an SM (square d =
+  // 2, n = 16, 5000 entries of 14 KB: 33 against 51 us; d = 3, n = 13, 3000 of 61
+  // KB: 197 against 260); an entry an SM takes twice the threads (d = 3, n = 18,
+  // 2000 entries of 156 KB: 426 against 582 us)
+  const long long half = device_info().smem_per_sm / 2 - 3072, need = r.group * 8LL;
+  if (need > device_info().max_smem_optin - 2048)
     return KRON_ERROR_NOT_SUPPORTED;
-  const int ng      = RECT_THREADS / r.GS;
+  while (r.GS < RECT_THREADS && RECT_THREADS / r.GS * need > half)
+    r.GS *= 2;
+  int threads = RECT_THREADS;
+  if (need > half)
+  {
+    fn      = reinterpret_cast<const void *>(&kron_rect_kernel<RECT_WIDE, 36, 1>);
+    threads = r.GS = RECT_WIDE;
+  }
+  const int ng      = threads / r.GS;
   const size_t smem = (size_t)ng * r.group * 8;
   int per_sm        = 1;
-  if (cached_occupancy(fn, RECT_THREADS, smem, &per_sm) != KRON_SUCCESS)
+  if (cached_occupancy(fn, threads, smem, &per_sm) != KRON_SUCCESS)
     return KRON_ERROR_LAUNCH;
   const long long work = (long long)p.eend - p.ebase;
   const long long grid =
       std::min<long long>((work + ng - 1) / ng, (long long)device_info().sms * per_sm);
   Params pp    = p;
   void *args[] = {&pp, &r};
-  return cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(RECT_THREADS), args, smem, stream) ==
+  return cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(threads), args, smem, stream) ==
                  cudaSuccess
              ? KRON_SUCCESS
              : KRON_ERROR_LAUNCH;

@@ -120,23 +120,27 @@ __device__ __forceinline__ void rect_innermost(const T *cur, T *nxt, const T *A,
   }
 }
 
-// Sizes beyond 8: one output element at a time (rare shapes, kept simple).
+// Sizes beyond 8: a thread an output element, so that short vectors with long
+// modes keep the whole group at work (a thread a fibre left one thread of 32 for
+// d = 1, n = 64, 32 of 128 for d = 2, n = 32: 100 entries 53 -> 12 and 95 -> 12
+// us, the larger groups of kron_rect.cu included).  Neighbouring threads read
+// neighbouring elements of x or of a column of the factor, and the same of the other.
 template <typename T>
 __device__ __noinline__ void rect_step_any(const T *cur, T *nxt, const T *A, int nq, int mq,
                                            int inner, unsigned magic, int nfib, int t, int GS)
 {
-  for (int f = t; f < nfib; f += GS)
+  const int total = nfib * mq;
+  for (int f = t; f < total; f += GS)
   {
-    const int o  = magic ? (int)__umulhi((unsigned)f, magic) : f;
-    const T *src = cur + f + o * inner * (nq - 1);
-    T *dst       = nxt + f + o * inner * (mq - 1);
-    for (int i = 0; i < mq; i++)
-    {
-      T z = T(0);
-      for (int j = 0; j < nq; j++)
-        z = fma(A[i + j * mq], src[j * inner], z);
-      dst[i * inner] = z;
-    }
+    // f = (o mq + i) inner + r
+    const int oi = magic ? (int)__umulhi((unsigned)f, magic) : f, r = f - oi * inner;
+    const int o  = oi / mq, i = oi - o * mq;
+    const T *src = cur + o * nq * inner + r, *a = A + i;
+    T z          = T(0);
+#pragma unroll 4
+    for (int j = 0; j < nq; j++)
+      z = fma(a[j * mq], src[j * inner], z);
+    nxt[f] = z;
   }
 }
 
