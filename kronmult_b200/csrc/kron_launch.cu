@@ -691,9 +691,10 @@ static bool variant_disabled(int v)
 }
 
 // FP32 d = 6, n = 6: a block an entry (resident) against a cluster of twelve
-// (slab), microseconds at 20 / 40 / 80 / 4096 entries: 19.8 / 20.5 / 20.9 /
-// 481 against 13.6 / 20.8 / 27.0 / 938.
-static bool prefer_resident(const Params &p) { return p.eend - p.ebase >= 40; }
+// (slab), microseconds at 20 / 42 / 50 / 60 / 64 / 84 / 4096 entries: 19.8 /
+// 20.5 / 20.5 / 20.5 / 20.5 / 20.5 / 481 against 13.6 / 18.5 / 19.4 / 20.5 /
+// 24.6 / 26.8 / 938.
+static bool prefer_resident(const Params &p) { return p.eend - p.ebase >= 60; }
 
 // FP64 d = 6, n = 6: the ring's two phases are a serial chain of about 40 us,
 // a cluster of twelve an entry (slab) finishes 21 entries in 14 us;
@@ -734,7 +735,9 @@ static bool prefer_pack(const Params &p)
 // n = 6: with exclusive outputs the square kernel's many warps are the better
 // use of 36 fibres an entry (d = 4, 8000 entries FP64 80 against 73, 600
 // entries 14.3 against 11.3; d = 5, 2000 entries FP64 123 against 121, FP32 72
-// against 55), but for d = 4 in FP32 (8000 entries: 45 against 49).
+// against 55), but for d = 4 in FP32 (8000 entries: 49 against 53, 20000: 100
+// against 113; only batches of 1500 to 8000 that stay in the L2 cache from call
+// to call are up to 4 us slower: 3500 20.5 against 16.8).
 // n = 8 and d = 5, n = 4: an entry alone on an SM is faster with 256 threads
 // than with 64 (n = 8 FP64 148 entries 12.3 against 9.2, 300: 16.4 against
 // 20.5; FP32 150: 12.3 against 9.2, 600: 14.3 against 18.4; d = 5, n = 4, 20:
