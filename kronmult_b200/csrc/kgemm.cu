@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(256)
 // the instructions of m8n8k4 at the same rate).  Four warps per entry, or one
 // (mm, nn <= 32), so that small entries fill an SM.  A warp holds TM x TN tiles
 // of 16 x 8 in fragments, 32 accumulators a lane: 32 x 32 of C, or 16 x 64, or 64 x
-// 16, whichever leaves the busiest warp least to do.
+// 16, as pick_dmma says.
 //
 // op(A) and op(B) are staged in shared memory line by line as they lie in
 // memory (lines of `len` contiguous elements), at a line stride of 4 mod 16
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(256)
 // still.
 //
 // Bound by HBM (64 x 64 x 64, 32768 entries: 4.3 GB, 0.66 ms; FP64 0.46).  Measured
-// there 1.20 -> 0.82 ms, 8 x 8 x 8 (60000 entries) 536 -> 52 us, 32 x 32 x 32 (60000)
+// there 1.20 -> 0.86 ms, 8 x 8 x 8 (60000 entries) 536 -> 52 us, 32 x 32 x 32 (60000)
 // 1017 -> 319 us, 58 x 35 x 29 (30000, beta = 0.5) 1382 -> 523 us, against one
 // entry a block whatever its size, loads, products and results in series, and two
 // divisions per copied element.
@@ -435,8 +435,13 @@ int pick_dmma(const DmArgs &p, cudaStream_t stream)
     return launch_dmma<OP, 1, 1, 2, 4, false>(p, stream);
   if (p.mm == 64 && p.nn == 64)
     return launch_dmma<OP, 2, 2, 2, 4, true>(p, stream);
-  // tiles of the busiest warp: two by two warps, four along the rows, four
-  // along the columns
+  // Tiles of the busiest warp: two by two warps of 2 x 4 tiles, four along the
+  // rows (1 x 8), four along the columns (4 x 2; rated as if its warps shared
+  // the tile columns evenly).  That decides at 3 x 4 tiles only, where two warps
+  // of 3 x 2 are faster than three of 1 x 4 (fewer shared-memory loads a product:
+  // 16 for 6 against 12 for 4 a K step; 20000 entries, beta = 1 / 0: 48 x 32 x 40
+  // 279 / 234 against 315 / 294 us, 40 x 30 x 64 372 / 330 against 401 / 375; only
+  // K = 8 is slower, 48 x 28 x 8 162 / 110 against 136 / 110).
   const int t22 = std::min(mt, 2) * std::min(nt, 4), t41 = nt, t14 = mt * ((nt + 3) / 4);
   if (t41 < t22 && t41 <= t14)
     return launch_dmma<OP, 4, 1, 1, 8, false>(p, stream);
@@ -454,7 +459,7 @@ int launch_kgemm(int op, int mm, int nn, int kk, double alpha, double *const *A,
   if (batch <= 0 || mm <= 0 || nn <= 0)
     return KRON_SUCCESS;
   // entries up to 64 x 64 x 64 (the reference tests' sizes) on the FP64
-  // tensor cores, one entry per block
+  // tensor cores, a block or (up to 32 x 32) a warp an entry
   if (mm <= DM_MAX && nn <= DM_MAX && kk <= DM_MAX && !std::getenv("KRON_KGEMM_CUDA_CORES"))
   {
     DmArgs p{};
