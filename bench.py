@@ -346,7 +346,7 @@ class BatchedSquare(Workload):
         """The precision sweep (the headline's config): FP64, FP32 and split
         (hi+lo FP32 arithmetic on FP64 data) at n = 4 and n = 6 on this
         batch, each timed like the headline (mean of 3 steps, L2 flushed
-        between) and checked against the reference's FP64 output of the same
+        between) and checked against the oracle's FP64 output of the same
         inputs; the headline's own case is timed again here for the speed-up
         ratios."""
         if not self.sweep:
@@ -382,8 +382,7 @@ class BatchedSquare(Workload):
                     del w
             out[f"n{n}_speedup_f32_over_f64"] = round(ms["f64"] / ms["f32"], 3)
             out[f"n{n}_speedup_split_over_f64"] = round(ms["f64"] / ms["split"], 3)
-        out["reference_output"] = ("oracle/_ref (the reference's OpenMP build, recursive "
-                                   "variant) on the same inputs, whole batch, FP64")
+        out["reference_output"] = f"{oracle_name()} on the same inputs, whole batch, FP64"
         return out
 
     def _repeated_apply(self, torch, w, reps=50):
@@ -946,20 +945,37 @@ def profile_key(args):
     return key
 
 
+def oracle_name():
+    """What the errors are measured against (oracle.reference_or_restatement)."""
+    import oracle
+
+    if oracle.Reference.available("recur"):
+        return "oracle/_ref (the reference's OpenMP build, recursive variant)"
+    return ("oracle/kron_oracle.c (a C restatement, pinned to the reference's vectors; the "
+            "reference's own build is not on this machine)")
+
+
 def read_profile_traffic(key):
     """Per-launch DRAM traffic of the dominant kernel from the committed ncu
-    summary (profiles/*.md line `traffic_bytes_per_launch[<key>]: <bytes>`)."""
+    summary (profiles/*.md line `traffic_bytes_per_launch[<key>]: <bytes>
+    <kernel>`), and the file."""
+    traffic, _kernel, src = read_profile_line(key)
+    return traffic, src
+
+
+def read_profile_line(key):
+    """The same with the kernel that the line names."""
     import glob
     import re
 
     for p in sorted(glob.glob(os.path.join(ROOT, "profiles", "*.md"))):
         with open(p) as f:
             for line in f:
-                m = re.match(rf"\s*traffic_bytes_per_launch\[{re.escape(key)}\]:\s*([0-9.eE+]+)",
-                             line)
+                m = re.match(rf"\s*traffic_bytes_per_launch\[{re.escape(key)}\]:\s*"
+                             r"([0-9.eE+]+)\s+(\w+)", line)
                 if m:
-                    return float(m.group(1)), os.path.relpath(p, ROOT)
-    return None, None
+                    return float(m.group(1)), m.group(2), os.path.relpath(p, ROOT)
+    return None, None, None
 
 
 class ClockSampler:
@@ -1216,7 +1232,7 @@ def run_ours(args, world, rank, local):
         value = world * flops * args.steps / sec / 1e9
         gbs = wl.alg_bytes() * args.steps / sec / 1e9
         per_launch_s = sec / (args.steps * wl.launches_per_step)
-        traffic, tsrc = read_profile_traffic(profile_key(args))
+        traffic, tkernel, tsrc = read_profile_line(profile_key(args))
         if args.config == 2 or args.config == 5:
             fp64 = measure_fp64_peak(torch)
             roof = {"bound": "tensor", "achieved": round(flops / wl.launches_per_step /
@@ -1238,9 +1254,10 @@ def run_ours(args, world, rank, local):
                     "traffic": traffic, "peak_source": f"MEASURED_PEAKS.json ({peak_src})"}
         if tsrc:
             roof["traffic_source"] = tsrc
+            roof["traffic_kernel"] = tkernel
         if wl.launches_per_step > 1:
             # achieved is the step's bytes over the step's time; traffic is
-            # the main launch's
+            # the main launch's (the ring's other one clears control words)
             roof["launches_per_step"] = wl.launches_per_step
         line = {"metric": METRIC, "value": round(value, 2), "unit": "GFLOP/s",
                 "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
