@@ -487,7 +487,9 @@ int sq_entries_max(int prec, int d, int n, bool merge)
 //
 // The slab kernel's clusters of 12 blocks fill whole GPCs only so far: on
 // B200 its 21 resident clusters hold 126 of the 148 SMs.  When the caller
-// passes a workspace, a share of the entries goes to the cluster two-phase
+// passes a workspace and the slab kernel runs all the same (the tuning table asks
+// for it, the ring kernel is disabled, or the workspace has less than the ring's
+// three vectors), a share of the entries goes to the cluster two-phase
 // kernel (clusters of 2) on a second stream, whose blocks take the idle SMs
 // while the slab kernel runs.  The share gives each idle SM SIDE_RATE of a
 // slab SM's entries (measured for 4096 entries of d = 6, n = 6: 1.59 ms

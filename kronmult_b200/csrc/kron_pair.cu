@@ -26,7 +26,9 @@
 // subnormals.
 //
 // Bound by latency with few warps an SM (n = 8: six, by shared memory and
-// registers; an instruction in 26% of a scheduler's cycles): batched FP64, before and after, d = 4, n = 8, 6000
+// registers; an instruction in 26% of a scheduler's cycles; FP64 d = 4, n = 8
+// spills 176 bytes a thread, 146 with sums in shared memory, d = 5, n = 7 300):
+// batched FP64, before and after, d = 4, n = 8, 6000
 // entries 324 -> 165 us (0.60 GB, HBM alone 92); d = 5, n = 7, 1000 entries 312
 // -> 129 (62); d = 6, n = 3, 10000 entries 132 -> 47 (27); 7200 entries of d = 4,
 // n = 8 on 800 outputs 332 -> 163; 36000 of d = 4, n = 5 on 4000 360 -> 89.

@@ -756,7 +756,9 @@ int launch_pipe_t(Params p, cudaStream_t stream)
 template <typename T>
 int pipe_pick(int d, int n, Params p, cudaStream_t s)
 {
-  // the (d, n) whose vectors are 4..64 KB in FP64 or FP32
+  // the (d, n) whose vectors are 4..64 KB in FP64 or FP32; all but (6, 4) and
+  // small batches of (5, 4) run only when the tuning table asks for this kernel
+  // or the pair kernel is disabled
   if (d == 6 && n == 3)
     return launch_pipe_t<T, 6, 3>(p, s);
   if (d == 5 && n == 4)

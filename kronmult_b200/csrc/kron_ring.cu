@@ -14,10 +14,11 @@
 // an item waits only for items that running blocks already hold: phase 2 for
 // its entry's K phase-1 parts, lag entries back (normally long done), and
 // phase 1 for the ring slot of W it writes, last read by the entry `slots`
-// positions back.  W is a ring of `slots` vectors, a few tens of MB that stay
-// in the L2 cache however large the batch; no cluster barriers, and every SM
-// works on both phases, so loads of x, math and adds into y overlap between
-// the blocks of an SM.
+// positions back.  W is a ring of `slots` vectors, a few tens of MB however
+// large the batch, most of it in the L2 cache (0.8 of its 3.1 GB of stores and
+// loads go to DRAM for 4096 entries of n = 6, 2.4 of 4.3 GB for 1024 of n = 8);
+// no cluster barriers, and every SM works on both phases, so loads of x, math
+// and adds into y overlap between the blocks of an SM.
 //
 // The control words (queue, abort, and per slot the parts done of each phase,
 // counted up over the slot's generations) lie in the workspace vector after
@@ -27,11 +28,11 @@
 // whole once its copies have landed; y of the parts not done is untouched.
 //
 // Measured against what ran before (the cluster two-phase kernel, whose W
-// goes through HBM and back: 9.35 against 6.9 GB for 1024 entries of n = 8;
+// goes through HBM and back: 9.35 against 6.87 GB for 1024 entries of n = 8;
 // n = 6: the slab-cluster kernel with its side kernel):
-//   n = 6, 4096 entries  1.40 -> 1.17 ms (HBM alone 0.70)
-//   n = 7, 256 entries   0.465 -> 0.241 ms (HBM alone 0.11)
-//   n = 8, 1024 entries with aliasing outputs  2.05 -> 1.71 ms (FP64 tensor
+//   n = 6, 4096 entries  1.40 -> 1.20 ms (HBM alone 0.70)
+//   n = 7, 256 entries   0.466 -> 0.250 ms (HBM alone 0.11)
+//   n = 8, 1024 entries with aliasing outputs  2.05 -> 1.79 ms (FP64 tensor
 //   pipe alone 0.70, HBM 0.98)
 #include <algorithm>
 #include <cstdint>
@@ -516,7 +517,8 @@ struct RingControl
 // A block is three such groups of four warps, which share nothing but the
 // control warps: three takers and a publisher.  One block an SM; the computing
 // warps take the registers that the control warps leave (160 of 128 + 128 / 3 a
-// thread: a fibre and a factor of n = 6 in FP64 are 144).
+// thread: a fibre and a factor of n = 6 in FP64 are 144).  Spill
+// stores are 48 bytes a thread there, 100 and 12 for n = 7, 8 in FP32.
 template <typename T, int N, int R_>
 struct RingShape
 {
